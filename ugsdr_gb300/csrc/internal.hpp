@@ -125,14 +125,20 @@ namespace ugsdr_gpu {
 		DevBuf cells;      // per (code, doppler) records
 		DevBuf params;     // per-job parameter arrays
 		DevBuf front;      // front-end output (resampled complex float) of jobs that need one
+		DevBuf folded;     // folded jobs: mixed blocks of the folded length
+		DevBuf fold_codes; // folded jobs: code spectra of the folded length
 		size_t reserved() const {
-			return samples.bytes + spectra.bytes + slab.bytes + cells.bytes + params.bytes + front.bytes;
+			return samples.bytes + spectra.bytes + slab.bytes + cells.bytes + params.bytes + front.bytes + folded.bytes +
+				fold_codes.bytes;
 		}
 		void set_stream(cudaStream_t s) {
-			samples.stream = spectra.stream = slab.stream = cells.stream = params.stream = front.stream = s;
+			samples.stream = spectra.stream = slab.stream = cells.stream = params.stream = front.stream = folded.stream =
+				fold_codes.stream = s;
 		}
 		void release() {
 			front.release();
+			folded.release();
+			fold_codes.release();
 			samples.release();
 			spectra.release();
 			slab.release();
