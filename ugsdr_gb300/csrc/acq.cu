@@ -6,6 +6,7 @@
 #include "acq_batched.cuh"
 #include "acq_cols_warp.cuh"
 #include "acq_folded.cuh"
+#include "acq_pairs.cuh"
 #include "dfe.cuh"
 #include "fft_plan.hpp"
 
@@ -142,12 +143,123 @@ namespace ugsdr_gpu {
 		return 0;
 	}
 
+	namespace {
+		// thread-instructions per point of an R-point DFT in registers: packed
+		// sums and multiply-adds of a prime's symmetric pairs, four for a
+		// composite's twiddle
+		double radix_cost(int r) {
+			if (is_prime(r)) {
+				const double h = (r - 1) / 2;
+				return r == 2 ? 1.0 : (7 * h + 2 * h * h) / r;
+			}
+			if (r == 4)
+				return 2.5;
+			const int a = smallest_factor(r), b = r / a;
+			return radix_cost(a) + radix_cost(b) + 4.0 * (1 - 1.0 / a) * (1 - 1.0 / b);
+		}
+
+		// issue rate that `threads`-thread CTAs of `bytes` shared memory and
+		// `regs` registers a thread sustain: resident warps w cover latency as
+		// w / (w + 6) (the warp kernels' 14 and 24 warps issue 55 and 67 %)
+		double pair_issue(ugsdr_ctx* ctx, int threads, int bytes, int regs) {
+			const int by_smem = static_cast<int>(ctx->smem_optin / (static_cast<size_t>(bytes) + 1024));
+			const int ctas = std::min({by_smem, 65536 / (regs * threads), 2048 / threads, 32});
+			const double w = ctas * threads / 32.0;
+			return w / (w + 6);
+		}
+
+		// The pair kernels' factors and tiles for a split: per candidate the
+		// thread-instructions per point of both passes (idle lanes of the last
+		// round of a pass included) over the issue rate its occupancy sustains.
+		// The constants beside the radix costs are the loads, stores, twiddles
+		// and index steps of each pass.
+		PairPlan pair_plan(ugsdr_ctx* ctx, int n1, int n2) {
+			PairPlan best;
+			double best_cost = 1e300;
+			auto pairs = [](int n) {
+				std::vector<std::pair<int, int>> out;
+				for (int a = 2; a <= 32; ++a)
+					if (n % a == 0 && n / a >= 2 && n / a <= 32)
+						out.push_back({a, n / a});
+				return out;
+			};
+			auto rounds = [](int work, int threads) { return (work + threads - 1) / threads; };
+			auto regs = [](int x, int y) { return std::max(x, y) <= 25 ? 80 : 128; };
+			for (const int shift : {2, 3}) {
+				const int cw = 1 << shift;
+				PairPlan cols, rows;
+				double c_cols = 1e300, c_rows = 1e300;
+				for (const auto& [a0, a1] : pairs(n1))
+					for (int t = 32; t <= kPairThreads; t += 32) {
+						const PairCols lay(a0, a1, cw);
+						if (lay.bytes > kPairSmem)
+							continue;
+						const double instr = t * (rounds(cw * a1, t) * a0 * (radix_cost(a0) + 3) + rounds(cw * a0, t) * a1 * (radix_cost(a1) + 15) + 20.0);
+						const double c = instr / (n1 * cw) / pair_issue(ctx, t, lay.bytes, regs(a0, a1)) * ((n2 + cw - 1) / cw * cw) / n2;
+						if (c < c_cols) {
+							c_cols = c;
+							cols.a0 = a0;
+							cols.a1 = a1;
+							cols.col_threads = t;
+						}
+					}
+				for (const auto& [b0, b1] : pairs(n2))
+					for (int rw = 1; rw <= 16; ++rw)
+						for (int t = 32; t <= kPairThreads; t += 32) {
+							const PairRows lay(b0, b1, rw, 1);
+							const PairRows full(b0, b1, rw, 0);
+							if (full.bytes > kPairSmem)
+								continue;
+							const double instr = t * (rounds(rw * b1, t) * b0 * (0.8 * radix_cost(b0) + 5) +
+								rounds(rw * b0, t) * b1 * (radix_cost(b1) + 18 + (b0 % cw ? 4 : 0)) + 20.0);
+							const double c = instr / (n2 * rw) / pair_issue(ctx, t, lay.bytes, regs(b0, b1)) * ((n1 + rw - 1) / rw * rw) / n1;
+							if (c < c_rows) {
+								c_rows = c;
+								rows.b0 = b0;
+								rows.b1 = b1;
+								rows.rw = rw;
+								rows.row_threads = t;
+							}
+						}
+				if (c_cols + c_rows < best_cost) {
+					best_cost = c_cols + c_rows;
+					best = PairPlan{cols.a0, cols.a1, rows.b0, rows.b1, shift, rows.rw, rows.row_threads, cols.col_threads};
+				}
+			}
+			return best;
+		}
+
+		bool pairable(int n) {
+			for (int a = 2; a <= 32; ++a)
+				if (n % a == 0 && n / a >= 2 && n / a <= 32)
+					return true;
+			return false;
+		}
+
+		// The rule's split, or where one of its halves is no product of two
+		// radices the split closest to square that is.
+		int preferred_split(ugsdr_ctx* ctx, int n) {
+			const int rule = rule_split(ctx, n);
+			if (rule == 0 || (pairable(rule) && pairable(n / rule)))
+				return rule;
+			for (int a = rule - 1; a >= 4; --a) {
+				if (n % a || !pairable(a) || !pairable(n / a))
+					continue;
+				if (split_fits(ctx, n, a, 4))
+					return a;
+				if (split_fits(ctx, n, n / a, 4))
+					return n / a;
+			}
+			return rule;
+		}
+	}
+
 	const LargePlan& get_large_plan(ugsdr_ctx* ctx, int n) {
 		auto it = ctx->large_plans.find(n);
 		if (it != ctx->large_plans.end())
 			return it->second;
 		const auto t = ctx->tiles.find(n);
-		const int best1 = t != ctx->tiles.end() && t->second.n1 > 0 ? t->second.n1 : rule_split(ctx, n);
+		const int best1 = t != ctx->tiles.end() && t->second.n1 > 0 ? t->second.n1 : preferred_split(ctx, n);
 		require(best1 > 0, "no four-step split for FFT size " + std::to_string(n), UGSDR_E_UNSUPPORTED);
 		LargePlan lp;
 		lp.n = n;
@@ -155,6 +267,8 @@ namespace ugsdr_gpu {
 		lp.n2 = n / best1;
 		lp.p1 = get_plan(ctx, lp.n1);
 		lp.p2 = get_plan(ctx, lp.n2);
+		if (pairable(lp.n1) && pairable(lp.n2))
+			lp.pair = pair_plan(ctx, lp.n1, lp.n2);
 		return ctx->large_plans[n] = lp;
 	}
 
@@ -265,8 +379,10 @@ namespace ugsdr_gpu {
 			if (t != ctx->tiles.end() && t->second.warp_cols == 0)
 				return 0;
 			int cw = 0;
-			with_cols_warp(n1, n2, [&](auto plan) { cw = decltype(plan)::CW; });
-			return cw;
+			if (with_cols_warp(n1, n2, [&](auto plan) { cw = decltype(plan)::CW; }))
+				return cw;
+			const PairPlan& pair = get_large_plan(ctx, n).pair;
+			return pair.a0 ? 1 << pair.cw_shift : 0;
 		}
 
 		BatchedParams batched_params(ugsdr_ctx* ctx, const AcqParams& base, int n) {
@@ -277,6 +393,8 @@ namespace ugsdr_gpu {
 			p.p2 = to_dev(lp.p2);
 			p.n1 = lp.n1;
 			p.n2 = lp.n2;
+			p.pair = PairSplit{lp.pair.a0, lp.pair.a1, lp.pair.b0, lp.pair.b1, lp.pair.cw_shift, lp.pair.rw, lp.pair.row_threads,
+				lp.pair.col_threads};
 			tile_shape(ctx, lp, p.cw, p.rw);
 			p.ld1 = lp.n1 | 1;  // odd column stride: the 8 columns of a tile fall in distinct banks
 			p.n2p = lp.n2;
@@ -499,11 +617,19 @@ namespace ugsdr_gpu {
 				launch_pair();
 				note_launch(ctx, 2);
 				if (s.fold_mode) {
-					fold_finish_kernel<<<p.rows, kBatchedThreads, 0, ctx->stream>>>(p);
+					fold_finish_kernel<><<<p.rows, kBatchedThreads, 0, ctx->stream>>>(p);
 					note_launch(ctx);
 				}
 			}
 		};
+		if (cw_blocked && !with_cols_warp(p.n1, p.n2, [](auto) {})) {
+			KernelTimer timer(ctx, "acq_inverse_large");
+			run_batches([&] {
+				launch_inv_rows_pair(p, half, ctx->stream);
+				launch_inv_cols_pair(p, ctx->stream);
+			});
+			return;
+		}
 		if (cw_blocked) {
 			// static row plan + warp-owned columns over the blocked B layout
 			with_large_ffts(p.n1, p.n2, [&](auto, auto f2) {
@@ -597,8 +723,8 @@ namespace ugsdr_gpu {
 				p.out = e.spectrum.as<float2>();
 				p.plan = to_dev(get_plan(ctx, n));
 				const size_t smem = 2 * sizeof(float2) * n;
-				set_smem(code_spectrum_kernel, smem);
-				code_spectrum_kernel<<<1, kThreads, smem, ctx->stream>>>(p);
+				set_smem(code_spectrum_kernel<>, smem);
+				code_spectrum_kernel<><<<1, kThreads, smem, ctx->stream>>>(p);
 				note_launch(ctx);
 			}
 			else {
@@ -919,9 +1045,9 @@ namespace ugsdr_gpu {
 			}
 			note_launch(ctx);
 			const size_t smem_i = 2 * sizeof(float2) * L.n + sizeof(float) * L.m;
-			set_smem(acq_inverse_kernel, smem_i);
+			set_smem(acq_inverse_kernel<>, smem_i);
 			KernelTimer timer(ctx, "acq_inverse");
-			acq_inverse_kernel<<<nd * L.n_codes, kThreads, smem_i, ctx->stream>>>(p);
+			acq_inverse_kernel<><<<nd * L.n_codes, kThreads, smem_i, ctx->stream>>>(p);
 			note_launch(ctx);
 		}
 		else {

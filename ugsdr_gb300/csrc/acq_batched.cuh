@@ -121,6 +121,13 @@ namespace ugsdr_gpu {
 	__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
 	__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
 
+	// Split of the pair kernels (acq_pairs.cuh): N1 = a0 a1, N2 = b0 b1 (a0 = 0:
+	// none), 1 << cw_shift columns and rw rows per CTA, threads of the row and
+	// column kernels
+	struct PairSplit {
+		int a0, a1, b0, b1, cw_shift, rw, row_threads, col_threads;
+	};
+
 	struct BatchedParams {
 		AcqParams base;         // n, k_blocks, n_doppler, n_codes, m, fold_mode, stat, one_sided, adders, lut, spectra, codes, cells
 		FftPlanDev p1, p2;      // N1-point, N2-point plans
@@ -130,6 +137,7 @@ namespace ugsdr_gpu {
 		int cw_shift;           // log2(cw)
 		int ld1;                // column-tile stride: N1 rounded up to odd (conflict-free smem)
 		// forward / code items
+		PairSplit pair;         // pair kernels only
 		int code_mode;          // 1: items are codes (chips -> spectra), 0: signal (Doppler, block)
 		int row_keep;           // signal spectra: elements k2 < row_keep of each row stored (0: all)
 		const float* chips;     // code mode: chips of code `item` at chips + item * chip_stride
@@ -1098,7 +1106,8 @@ namespace ugsdr_gpu {
 	}
 
 	// folded rows: acc (fold 1) or |complex fold| summed over blocks (fold 2) -> cell; grid: rows
-	static __global__ void __launch_bounds__(256) fold_finish_kernel(BatchedParams p) {
+	template <class = void>
+	__global__ void __launch_bounds__(256) fold_finish_kernel(BatchedParams p) {
 		const AcqParams& q = p.base;
 		const int lrow = blockIdx.x;
 		const int m = q.m;

@@ -13,8 +13,8 @@
 //                          scale -> |.| or |.|^2 -> fold -> accumulate over the
 //                          K blocks in shared memory -> first-max / mean / std
 //                          -> one 16-byte cell record to HBM
-// plus acq_select_kernel (per code: first strictly greater level over Doppler,
-// fse.hpp:265).
+// (the per-code choice over Doppler, first strictly greater level, fse.hpp:265,
+// is made on the host from the cells).
 #pragma once
 
 #include "fft_core.cuh"
@@ -121,7 +121,8 @@ namespace ugsdr_gpu {
 		return v;
 	}
 
-	static __global__ void code_spectrum_kernel(CodeSpecParams p) {
+	template <class = void>
+	__global__ void code_spectrum_kernel(CodeSpecParams p) {
 		extern __shared__ float2 smem[];
 		float2* a = smem;
 		float2* b = smem + p.plan.n;
@@ -276,7 +277,8 @@ namespace ugsdr_gpu {
 		}
 	}
 
-	static __global__ void acq_inverse_kernel(AcqParams p) {
+	template <class = void>
+	__global__ void acq_inverse_kernel(AcqParams p) {
 		extern __shared__ float2 smem[];
 		float2* a = smem;
 		float2* b = smem + p.n;
@@ -325,21 +327,5 @@ namespace ugsdr_gpu {
 			__syncthreads();
 		}
 		reduce_cell(acc, p.m, p.cells + static_cast<size_t>(c) * p.n_doppler + p.d_base + d);
-	}
-
-	// per code: keep the first Doppler with a strictly greater level (fse.hpp:265)
-	static __global__ void acq_select_kernel(const AcqCellDev* cells, int n_codes, int n_doppler, int* best_bin) {
-		const int c = blockIdx.x * blockDim.x + threadIdx.x;
-		if (c >= n_codes)
-			return;
-		const AcqCellDev* row = cells + static_cast<size_t>(c) * n_doppler;
-		int best = 0;
-		float lvl = row[0].level;
-		for (int d = 1; d < n_doppler; ++d)
-			if (lvl < row[d].level) {
-				lvl = row[d].level;
-				best = d;
-			}
-		best_bin[c] = best;
 	}
 }

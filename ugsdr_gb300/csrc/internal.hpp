@@ -80,10 +80,18 @@ namespace ugsdr_gpu {
 		const float2* tw = nullptr;
 	};
 
+	// Factors and tiles of the pair kernels for a split (acq.cu pair_plan;
+	// a0 = 0: a half of the split is not a product of two radices).
+	struct PairPlan {
+		int a0 = 0, a1 = 0, b0 = 0, b1 = 0;
+		int cw_shift = 0, rw = 0, row_threads = 0, col_threads = 0;
+	};
+
 	// Four-step split N = N1 * N2 for sizes above the single-CTA limit.
 	struct LargePlan {
 		int n = 0;
 		int n1 = 0, n2 = 0;
+		PairPlan pair;
 		FftPlanDesc p1, p2;    // N1-point and N2-point plans (the inter-step twiddles are computed in the kernels)
 	};
 

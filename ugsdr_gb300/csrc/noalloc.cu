@@ -187,7 +187,7 @@ extern "C" int ugsdr_acquire_static(void* cuda_stream, const ugsdr_static_job* j
 	plan.tw = tw;
 
 	// every kernel's shared-memory opt-in is set before the first launch
-	bool smem_set = smem_ok(static_code_spectra_kernel, smem_f) && smem_ok(acq_inverse_kernel, smem_i);
+	bool smem_set = smem_ok(static_code_spectra_kernel, smem_f) && smem_ok(acq_inverse_kernel<>, smem_i);
 	switch (job->sample_type) {
 	case UGSDR_SAMPLES_CF32: smem_set = smem_set && smem_ok(acq_forward_kernel<UGSDR_SAMPLES_CF32>, smem_f); break;
 	case UGSDR_SAMPLES_CI8: smem_set = smem_set && smem_ok(acq_forward_kernel<UGSDR_SAMPLES_CI8>, smem_f); break;
@@ -233,7 +233,7 @@ extern "C" int ugsdr_acquire_static(void* cuda_stream, const ugsdr_static_job* j
 	case UGSDR_SAMPLES_CI16: acq_forward_kernel<UGSDR_SAMPLES_CI16><<<grid_f, kThreads, smem_f, stream>>>(p); break;
 	default: acq_forward_kernel<UGSDR_SAMPLES_RI8><<<grid_f, kThreads, smem_f, stream>>>(p); break;
 	}
-	acq_inverse_kernel<<<static_cast<int>(grid_inv), kThreads, smem_i, stream>>>(p);
+	acq_inverse_kernel<><<<static_cast<int>(grid_inv), kThreads, smem_i, stream>>>(p);
 	if (cudaGetLastError() != cudaSuccess)
 		return UGSDR_E_CUDA;
 	return UGSDR_OK;
