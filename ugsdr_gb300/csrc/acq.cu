@@ -158,22 +158,27 @@ namespace ugsdr_gpu {
 			return radix_cost(a) + radix_cost(b) + 4.0 * (1 - 1.0 / a) * (1 - 1.0 / b);
 		}
 
-		// issue rate that `threads`-thread CTAs of `bytes` shared memory and
-		// `regs` registers a thread sustain: resident warps w cover latency as
-		// w / (w + 6) (the warp kernels' 14 and 24 warps issue 55 and 67 %)
-		double pair_issue(ugsdr_ctx* ctx, int threads, int bytes, int regs) {
-			const int by_smem = static_cast<int>(ctx->smem_optin / (static_cast<size_t>(bytes) + 1024));
+		// What `threads`-thread CTAs of `bytes` shared memory and `regs` registers
+		// a thread lose to latency: w resident warps run at w / (w + half) of the
+		// rate that enough of them would.
+		double pair_latency(int threads, int bytes, int regs, double half) {
+			const int by_smem = (kPairSmem + 1024) / (bytes + 1024);
 			const int ctas = std::min({by_smem, 65536 / (regs * threads), 2048 / threads, 32});
 			const double w = ctas * threads / 32.0;
-			return w / (w + 6);
+			return (w + half) / w;
 		}
 
 		// The pair kernels' factors and tiles for a split: per candidate the
 		// thread-instructions per point of both passes (idle lanes of the last
-		// round of a pass included) over the issue rate its occupancy sustains.
-		// The constants beside the radix costs are the loads, stores, twiddles
-		// and index steps of each pass.
-		PairPlan pair_plan(ugsdr_ctx* ctx, int n1, int n2) {
+		// round of a pass included) times what its occupancy loses.  The weights
+		// beside the radix costs (18 and 30 a point in the row kernel's passes, 22
+		// and 30 in the column kernel's, 21 and 16 warps, 1.5 and 1.4 hundredths
+		// of a ps) are a fit to 340 measured shapes of ten sizes from 16,384 to
+		// 332,500 points; of the shapes measured for one split the fit's choice is
+		// 1.4 % (rows) and 3.4 % (columns) slower than the fastest on average.
+		// More than eight rows, or more than 192 threads, per row CTA were never
+		// the fastest.
+		PairPlan pair_plan(int n1, int n2) {
 			PairPlan best;
 			double best_cost = 1e300;
 			auto pairs = [](int n) {
@@ -194,8 +199,8 @@ namespace ugsdr_gpu {
 						const PairCols lay(a0, a1, cw);
 						if (lay.bytes > kPairSmem)
 							continue;
-						const double instr = t * (rounds(cw * a1, t) * a0 * (radix_cost(a0) + 3) + rounds(cw * a0, t) * a1 * (radix_cost(a1) + 15) + 20.0);
-						const double c = instr / (n1 * cw) / pair_issue(ctx, t, lay.bytes, regs(a0, a1)) * ((n2 + cw - 1) / cw * cw) / n2;
+						const double instr = t * (rounds(cw * a1, t) * a0 * (radix_cost(a0) + 22) + rounds(cw * a0, t) * a1 * (radix_cost(a1) + 30));
+						const double c = 1.4 * instr / (n1 * cw) * pair_latency(t, lay.bytes, regs(a0, a1), 16.0) * ((n2 + cw - 1) / cw * cw) / n2;
 						if (c < c_cols) {
 							c_cols = c;
 							cols.a0 = a0;
@@ -204,15 +209,14 @@ namespace ugsdr_gpu {
 						}
 					}
 				for (const auto& [b0, b1] : pairs(n2))
-					for (int rw = 1; rw <= 16; ++rw)
-						for (int t = 32; t <= kPairThreads; t += 32) {
+					for (const int rw : {4, 8})
+						for (int t = 32; t <= 192; t += 32) {
 							const PairRows lay(b0, b1, rw, 1);
 							const PairRows full(b0, b1, rw, 0);
 							if (full.bytes > kPairSmem)
 								continue;
-							const double instr = t * (rounds(rw * b1, t) * b0 * (0.8 * radix_cost(b0) + 5) +
-								rounds(rw * b0, t) * b1 * (radix_cost(b1) + 18 + (b0 % cw ? 4 : 0)) + 20.0);
-							const double c = instr / (n2 * rw) / pair_issue(ctx, t, lay.bytes, regs(b0, b1)) * ((n1 + rw - 1) / rw * rw) / n1;
+							const double instr = t * (rounds(rw * b1, t) * b0 * (0.8 * radix_cost(b0) + 18) + rounds(rw * b0, t) * b1 * (radix_cost(b1) + 30));
+							const double c = 1.5 * instr / (n2 * rw) * pair_latency(t, lay.bytes, regs(b0, b1), 21.0) * ((n1 + rw - 1) / rw * rw) / n1;
 							if (c < c_rows) {
 								c_rows = c;
 								rows.b0 = b0;
@@ -268,7 +272,7 @@ namespace ugsdr_gpu {
 		lp.p1 = get_plan(ctx, lp.n1);
 		lp.p2 = get_plan(ctx, lp.n2);
 		if (pairable(lp.n1) && pairable(lp.n2))
-			lp.pair = pair_plan(ctx, lp.n1, lp.n2);
+			lp.pair = pair_plan(lp.n1, lp.n2);
 		return ctx->large_plans[n] = lp;
 	}
 

@@ -74,11 +74,15 @@ namespace ugsdr_gpu {
 		}
 	};
 	struct PairRows {
-		int pad, ldb, live, lds, tws;  // live inputs of a pass-0 butterfly, staged code elements per row
+		int pad, ldb, live, lds, tws;  // tile row stride, live inputs of a pass-0 butterfly, staged code elements per row
 		int cs_at, tw_at, seeds_at, bytes;
+		// rw: a power of two >= 4.  Pass 1's half-warps read rw rows x 16 / rw
+		// neighbours: a row stride of 16 / rw modulo 16 puts them in distinct banks.
 		UG_HD PairRows(int b0, int b1, int rw, int half) {
 			pad = (b0 & 1) ^ 1;
 			ldb = (b0 + pad) * b1;
+			const int want = rw < 16 ? 16 / rw : 1;
+			ldb += (want - ldb % 16 + 16) % 16;
 			live = half ? b0 / 2 + 1 : b0;
 			lds = live * b1;
 			tws = (b1 - 1) | 1;
@@ -127,7 +131,8 @@ namespace ugsdr_gpu {
 		const float2* xg = q.spectra + static_cast<size_t>(d) * q.k_blocks * n + static_cast<size_t>(r0) * n2;
 		const size_t out_block = static_cast<size_t>(n1) * p.n2p;
 		float2* out = p.bbuf + static_cast<size_t>(lrow) * q.k_blocks * out_block + (r0 << cw_shift);
-		const float inv_b1 = 1.0f / static_cast<float>(b1), inv_b0 = 1.0f / static_cast<float>(b0);
+		const float inv_b1 = 1.0f / static_cast<float>(b1);
+		const int rw_shift = 31 - __clz(p.pair.rw);
 		const int chunk_elems = n1 << cw_shift;
 		for (int blk = 0; blk < q.k_blocks; ++blk, xg += n, out += out_block) {
 			// pass 0: radix b0, input k2 = j + r b1, j < b1
@@ -161,8 +166,12 @@ namespace ugsdr_gpu {
 			with_radix<MAXR>(b1, [&](auto rc) {
 				constexpr int R = decltype(rc)::value;
 				const int stride = b0 + lay.pad;
-				for (int u = threadIdx.x; u < rw * b0; u += blockDim.x) {
-					const int f = fdiv(u, inv_b0), j = u - f * b0;
+				for (int u = threadIdx.x; u < b0 << rw_shift; u += blockDim.x) {
+					// rows fastest: a warp's stores of one output are whole
+					// 32-byte pieces of adjacent rows, 128-byte lines of B
+					const int f = u & (p.pair.rw - 1), j = u >> rw_shift;
+					if (f >= rw)
+						continue;
 					const float2* src = b + f * lay.ldb + j;
 					const float2* wk = tw + j * lay.tws - 1;
 					float2 v[R];
