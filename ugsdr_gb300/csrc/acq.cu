@@ -6,7 +6,8 @@
 #include "acq_batched.cuh"
 #include "acq_cols_warp.cuh"
 #include "acq_folded.cuh"
-#include "acq_pairs.cuh"
+#include "acq_pairs_fwd.cuh"
+#include "acq_small.cuh"
 #include "dfe.cuh"
 #include "fft_plan.hpp"
 
@@ -276,6 +277,20 @@ namespace ugsdr_gpu {
 		return ctx->large_plans[n] = lp;
 	}
 
+	// Whether an unfolded search of block size n runs the four-step kernels: all
+	// that one CTA cannot hold, and of those it can the ones that leave a single
+	// CTA per SM (20 bytes a point), where their split suits the pair kernels.
+	// Measured, 32 codes x 21 bins x 10 blocks: 10,230 points 1382 -> 528 us a
+	// search, 8,184 1172 -> 515, 6,944 811 -> 427; at 4,092, where two CTAs share
+	// an SM, 376 -> 342 with every call of few rows slower (four launches, not two).
+	bool runs_four_step(ugsdr_ctx* ctx, int n) {
+		if (!fits_single_cta(ctx, n))
+			return true;
+		if (static_cast<size_t>(n) * 20 + 2048 <= ctx->smem_optin / 2)
+			return false;
+		return rule_split(ctx, n) != 0 && get_large_plan(ctx, n).pair.a0 != 0;
+	}
+
 	namespace {
 		constexpr int kBatchedThreads = 256;
 
@@ -449,7 +464,23 @@ namespace ugsdr_gpu {
 			kernel<<<items * chunks_of(p.n2, p.cw), threads, smem, ctx->stream>>>(p);
 		}
 
+		// splits with compile-time sub-FFT plans for the inverse
+		bool has_static_plan(int n1, int n2) { return (n1 == 200 && n2 == 250) || (n1 == 400 && n2 == 500); }
+
 		void launch_forward(ugsdr_ctx* ctx, int sample_type, const BatchedParams& p, int items) {
+			// signal items (and the per-op DFT's): the pair kernels, measured at 41
+			// bins x 40 blocks of 50,000 points 525 us against 595 for the
+			// compile-time 200 x 250 plans, x 10 of 40,920 247 against 365 for the
+			// runtime plans
+			if (!p.code_mode && p.pair.a0 && !std::getenv("UGSDR_NO_WARP_FWD_ROWS")) {
+				auto cols = sample_type == UGSDR_SAMPLES_CF32 ? launch_fwd_cols_pair_cf32
+					: sample_type == UGSDR_SAMPLES_CI8 ? launch_fwd_cols_pair_ci8
+					: sample_type == UGSDR_SAMPLES_CI16 ? launch_fwd_cols_pair_ci16 : launch_fwd_cols_pair_ri8;
+				cols(p, items, ctx->stream);
+				launch_fwd_rows_pair(p, items, ctx->stream);
+				note_launch(ctx, 2);
+				return;
+			}
 			with_large_ffts(p.n1, p.n2, [&](auto f1, auto f2) {
 				using F1 = decltype(f1);
 				using F2 = decltype(f2);
@@ -583,7 +614,9 @@ namespace ugsdr_gpu {
 		// only the lower part of each signal-spectrum row: only that is stored
 		const int wr = warp_rows_mode(ctx, s.n);
 		const bool half = base.one_sided != 0 && !std::getenv("UGSDR_NO_PRUNE");
-		if (cw_blocked && wr != 0 && half)
+		if (cw_blocked && half && !has_static_plan(p.n1, p.n2))
+			p.row_keep = PairRows(p.pair.b0, p.pair.b1, p.pair.rw, 1).lds;
+		else if (cw_blocked && wr != 0 && half)
 			with_large_ffts(p.n1, p.n2, [&](auto, auto f2) {
 				using F2 = decltype(f2);
 				if constexpr (F2::kHooked && F2::kRowsCompact)
@@ -626,7 +659,7 @@ namespace ugsdr_gpu {
 				}
 			}
 		};
-		if (cw_blocked && !with_cols_warp(p.n1, p.n2, [](auto) {})) {
+		if (cw_blocked && !has_static_plan(p.n1, p.n2)) {
 			KernelTimer timer(ctx, "acq_inverse_large");
 			run_batches([&] {
 				launch_inv_rows_pair(p, half, ctx->stream);
@@ -747,6 +780,7 @@ namespace ugsdr_gpu {
 		bool large = false;
 		bool front = false;   // device front end (mix at the input rate + resample) first
 		int folds = 1;        // F > 1: the block of F n samples is folded to n before the transforms
+		bool own_codes = false;  // code spectra of another length or layout than the handles'
 		float code_scale = 1.f;  // folded jobs: factor on the code spectra
 		ResamplePlan rs{};
 	};
@@ -853,7 +887,8 @@ namespace ugsdr_gpu {
 					job.n_samples) > 0, "BBP DDC captures need a whole-kHz rate and whole 1 ms epochs");
 			if (L.fold_mode != 0)
 				fold_first(ctx, job, L);
-			L.large = !fits_single_cta(ctx, L.n);
+			L.large = L.fold_mode == 0 ? runs_four_step(ctx, L.n) : !fits_single_cta(ctx, L.n);
+			L.own_codes = L.folds > 1 || ctx->codes[job.codes[0]]->large != L.large;
 			return L;
 		}
 
@@ -927,8 +962,8 @@ namespace ugsdr_gpu {
 	}
 
 	// The folded length's code spectra C[q F] in the layout its transforms read.
-	void launch_fold_codes(ugsdr_ctx* ctx, const ugsdr_acq_job& job, int m, int folds, float scale, float2* out) {
-		const int n1_out = fits_single_cta(ctx, m) ? 0 : get_large_plan(ctx, m).n1;
+	void launch_fold_codes(ugsdr_ctx* ctx, const ugsdr_acq_job& job, int m, bool large, int folds, float scale, float2* out) {
+		const int n1_out = large ? get_large_plan(ctx, m).n1 : 0;
 		FoldCodesParams p{};
 		p.m = m;
 		p.folds = folds;
@@ -961,6 +996,67 @@ namespace ugsdr_gpu {
 	}
 
 	namespace {
+		// The single-CTA kernels' plan of block size n: radices, the pass twiddle
+		// tables (per pass s >= 1 W_N^{r k N / (NS R)} at [r - 1][k]), threads and
+		// CTAs per row.  n_pass = 0: a size those kernels don't take (a lone
+		// pass, or tiles beyond shared memory).
+		SmallPlan small_plan(ugsdr_ctx* ctx, int n, int rows, int k_blocks, bool one_sided) {
+			const FftPlanDesc& d = get_plan(ctx, n);
+			SmallPlan p{};
+			p.n = n;
+			p.n_pass = d.n_pass;
+			for (int s = 0; s < d.n_pass; ++s)
+				p.radix[s] = d.radix[s];
+			if (d.n_pass < 2 || small_inv_bytes(p) > kSmallSmem) {
+				p.n_pass = 0;
+				return p;
+			}
+			auto& slot = ctx->pass_tables[n];
+			if (!slot) {
+				std::vector<float2> t;
+				const double two_pi = 2.0 * 3.14159265358979323846;
+				int ns = d.radix[0];
+				for (int s = 1; s < d.n_pass; ++s) {
+					const int step = n / (ns * d.radix[s]);
+					for (int r = 1; r < d.radix[s]; ++r)
+						for (int k = 0; k < ns; ++k) {
+							const double a = two_pi * static_cast<double>(static_cast<int64_t>(r) * k * step % n) / n;
+							t.push_back(c2(static_cast<float>(std::cos(a)), static_cast<float>(-std::sin(a))));
+						}
+					ns *= d.radix[s];
+				}
+				auto buf = std::make_unique<DevBuf>();
+				buf->reserve(sizeof(float2) * t.size());
+				UG_CUDA(cudaMemcpy(buf->ptr, t.data(), sizeof(float2) * t.size(), cudaMemcpyHostToDevice));
+				UG_CUDA(cudaStreamSynchronize(nullptr));  // in place before any stream reads it
+				slot = std::move(buf);
+			}
+			p.tables = slot->as<float2>();
+			// threads: the most (up to 256) whose idle lanes in the passes' last
+			// rounds cost no more than a tenth over the best choice
+			auto cost = [&](int t) {
+				double c = 0;
+				for (int s = 0; s < p.n_pass; ++s)
+					c += static_cast<double>((n / p.radix[s] + t - 1) / t) * t * p.radix[s];
+				return c;
+			};
+			double best = 1e300;
+			for (int t = 64; t <= kSmallThreads; t += 32)
+				best = std::min(best, cost(t));
+			p.threads = 64;
+			for (int t = 64; t <= kSmallThreads; t += 32)
+				if (cost(t) <= 1.1 * best)
+					p.threads = t;
+			// rows that leave CTA slots empty: the K blocks of a row go to several
+			// CTAs (a cluster of eight at most), the same number of blocks each
+			const int regs = !one_sided ? 255 : *std::max_element(p.radix, p.radix + p.n_pass) <= 25 ? 80 : 128;
+			const int per_sm = std::max(1, std::min(kSmallSmem / (small_inv_bytes(p) + 1024), 65536 / (regs * p.threads)));
+			int split = std::min({8, k_blocks, std::max(1, ctx->sm_count * per_sm / std::max(rows, 1))});
+			split = (k_blocks + (k_blocks + split - 1) / split - 1) / ((k_blocks + split - 1) / split);
+			p.split = split;
+			return p;
+		}
+
 		// single-CTA block sizes with a compile-time plan (4000: 1 ms at 4 MHz)
 		template <class Fn>
 		bool with_small_fft(int n, Fn&& fn) {
@@ -1022,6 +1118,22 @@ namespace ugsdr_gpu {
 		if (!L.large && L.fold_mode == 0 && L.m == L.n && L.n == 4000) {
 			with_small_fft(L.n, [&](auto f) { launch_small_static<decltype(f)>(ctx, sample_type, fwd, p, nd, L.k, L.n_codes); });
 			return;
+		}
+		if (!L.large && L.fold_mode == 0) {
+			const SmallPlan plan = small_plan(ctx, L.n, nd * L.n_codes, L.k, p.one_sided != 0);
+			if (plan.n_pass) {
+				{
+					KernelTimer timer(ctx, "acq_forward");
+					const bool narrow = sample_type == UGSDR_SAMPLES_CI8 || sample_type == UGSDR_SAMPLES_RI8;
+					(narrow ? launch_fwd_small_8bit : launch_fwd_small_wide)(fwd, plan, sample_type, nd * L.k, ctx->stream);
+				}
+				note_launch(ctx);
+				KernelTimer timer(ctx, "acq_inverse");
+				const bool low = p.one_sided && *std::max_element(plan.radix, plan.radix + plan.n_pass) <= 25;
+				(low ? launch_inv_small25 : launch_inv_small32)(p, plan, nd * L.n_codes, ctx->stream);
+				note_launch(ctx);
+				return;
+			}
 		}
 		if (!L.large) {
 			const size_t smem_f = 2 * sizeof(float2) * L.n;
@@ -1106,10 +1218,10 @@ namespace ugsdr_gpu {
 		}
 
 		// folded jobs: the folded blocks of one Doppler chunk, and the code
-		// spectra of the folded length
+		// spectra of the folded length (or only of the other layout)
 		size_t folded_bytes(const JobLaunch& L) { return L.folds > 1 ? spectra_bytes(L) : 0; }
-		size_t folded_codes_bytes(const JobLaunch& L) {
-			return L.folds > 1 ? (sizeof(float2) * static_cast<size_t>(L.n) * L.n_codes + 255) / 256 * 256 : 0;
+		size_t own_codes_bytes(const JobLaunch& L) {
+			return L.own_codes ? (sizeof(float2) * static_cast<size_t>(L.n) * L.n_codes + 255) / 256 * 256 : 0;
 		}
 
 		BatchSizes size_batch(ugsdr_ctx* ctx, const ugsdr_acq_job* jobs, int n_jobs) {
@@ -1129,7 +1241,7 @@ namespace ugsdr_gpu {
 				s.cells += static_cast<size_t>(L.n_codes) * L.grid.size();
 				s.front += front_bytes(L);
 				s.folded = std::max(s.folded, folded_bytes(L));
-				s.fold_codes += folded_codes_bytes(L);
+				s.fold_codes += own_codes_bytes(L);
 				s.params += (L.grid.size() * sizeof(uint32_t) + L.n_codes * sizeof(void*) + L.n_codes * sizeof(int) + 512) / 256 * 256;
 				if (L.large)
 					s.slab = std::max(s.slab, batched_scratch_bytes(ctx, shape_of(L)));
@@ -1164,10 +1276,10 @@ namespace ugsdr_gpu {
 			ws.slab.reserve(sizes.slab);
 		if (sizes.front)
 			ws.front.reserve(sizes.front);
-		if (sizes.folded) {
+		if (sizes.folded)
 			ws.folded.reserve(sizes.folded);
+		if (sizes.fold_codes)
 			ws.fold_codes.reserve(sizes.fold_codes);
-		}
 		StreamSwap swap(ctx, stream);
 
 		// stage parameters and host samples
@@ -1204,12 +1316,12 @@ namespace ugsdr_gpu {
 			size_t o = (L.adders.size() * sizeof(uint32_t) + 15) / 16 * 16;
 			fc_offsets[j] = fc_off;
 			for (int c = 0; c < L.n_codes; ++c) {
-				const float2* ptr = L.folds > 1
+				const float2* ptr = L.own_codes
 					? reinterpret_cast<const float2*>(ws.fold_codes.as<char>() + fc_off) + static_cast<size_t>(c) * L.n
 					: ctx->codes[job.codes[c]]->spectrum.as<float2>();
 				std::memcpy(hp + o + c * sizeof(void*), &ptr, sizeof(void*));
 			}
-			fc_off += folded_codes_bytes(L);
+			fc_off += own_codes_bytes(L);
 			p_off += (L.grid.size() * sizeof(uint32_t) + L.n_codes * sizeof(void*) + L.n_codes * sizeof(int) + 512) / 256 * 256;
 			c_offsets[j] = c_off;
 			c_off += static_cast<size_t>(L.n_codes) * L.grid.size();
@@ -1230,8 +1342,8 @@ namespace ugsdr_gpu {
 				job.sample_type = UGSDR_SAMPLES_CF32;
 				job.frontend_frequency = 0.0;
 			}
-			if (L.folds > 1)
-				launch_fold_codes(ctx, job, L.n, L.folds, L.code_scale,
+			if (L.own_codes)
+				launch_fold_codes(ctx, job, L.n, L.large, L.folds, L.code_scale,
 					reinterpret_cast<float2*>(ws.fold_codes.as<char>() + fc_offsets[j]));
 			char* dp = ws.params.as<char>() + p_offsets[j];
 			auto* adders = reinterpret_cast<uint32_t*>(dp);
@@ -1458,7 +1570,7 @@ namespace ugsdr_gpu {
 		std::map<int, std::vector<ugsdr_acq_job>> by_size;
 		for (int j = 0; j < n_jobs; ++j) {
 			const JobLaunch L = validate(ctx, jobs[j]);
-			if (L.large)
+			if (L.large && !fits_single_cta(ctx, L.n))
 				by_size[L.n].push_back(jobs[j]);
 		}
 		for (const auto& [n, all] : by_size) {
@@ -1534,7 +1646,7 @@ int ugsdr_code_put(ugsdr_ctx* ctx, const float* chips, size_t n_chips, size_t re
 		auto e = std::make_unique<CodeEntry>();
 		e->n = samples;
 		e->spectrum_mode = spectrum_mode;
-		e->large = !fits_single_cta(ctx, static_cast<int>(samples));
+		e->large = runs_four_step(ctx, static_cast<int>(samples));
 		build_code_spectrum(ctx, *e, chips, n_chips, repeats, sign_mask, sign_segment);
 		e->chips.assign(chips, chips + n_chips);
 		e->repeats = repeats;

@@ -1,0 +1,8 @@
+// Forward pair column kernel, cf32 samples.
+#include "acq_pairs_fwd.cuh"
+
+namespace ugsdr_gpu {
+	void launch_fwd_cols_pair_cf32(const BatchedParams& p, int items, cudaStream_t stream) {
+		launch_fwd_cols_pair<UGSDR_SAMPLES_CF32>(p, items, stream);
+	}
+}

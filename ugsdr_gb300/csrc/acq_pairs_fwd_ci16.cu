@@ -1,0 +1,8 @@
+// Forward pair column kernel, ci16 samples.
+#include "acq_pairs_fwd.cuh"
+
+namespace ugsdr_gpu {
+	void launch_fwd_cols_pair_ci16(const BatchedParams& p, int items, cudaStream_t stream) {
+		launch_fwd_cols_pair<UGSDR_SAMPLES_CI16>(p, items, stream);
+	}
+}

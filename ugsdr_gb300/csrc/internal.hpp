@@ -134,7 +134,7 @@ namespace ugsdr_gpu {
 		DevBuf params;     // per-job parameter arrays
 		DevBuf front;      // front-end output (resampled complex float) of jobs that need one
 		DevBuf folded;     // folded jobs: mixed blocks of the folded length
-		DevBuf fold_codes; // folded jobs: code spectra of the folded length
+		DevBuf fold_codes; // code spectra of the folded length or of another layout than the handles'
 		size_t reserved() const {
 			return samples.bytes + spectra.bytes + slab.bytes + cells.bytes + params.bytes + front.bytes + folded.bytes +
 				fold_codes.bytes;
@@ -168,6 +168,7 @@ struct ugsdr_ctx {
 	std::map<int, std::unique_ptr<ugsdr_gpu::DevBuf>> twiddles;
 	std::map<int, ugsdr_gpu::FftPlanDesc> plans;
 	std::map<int, ugsdr_gpu::LargePlan> large_plans;
+	std::map<int, std::unique_ptr<ugsdr_gpu::DevBuf>> pass_tables;  // single-CTA kernels: pass twiddles per size
 	std::map<int, ugsdr_gpu::TileChoice> tiles;  // per block size (ugsdr_tile_set / ugsdr_autotune)
 
 	// code spectra
