@@ -476,8 +476,8 @@ namespace ugsdr_gpu {
 				auto cols = sample_type == UGSDR_SAMPLES_CF32 ? launch_fwd_cols_pair_cf32
 					: sample_type == UGSDR_SAMPLES_CI8 ? launch_fwd_cols_pair_ci8
 					: sample_type == UGSDR_SAMPLES_CI16 ? launch_fwd_cols_pair_ci16 : launch_fwd_cols_pair_ri8;
-				cols(p, items, ctx->stream);
-				launch_fwd_rows_pair(p, items, ctx->stream);
+				cols(p, items, ctx->sm_count, ctx->stream);
+				launch_fwd_rows_pair(p, items, ctx->sm_count, ctx->stream);
 				note_launch(ctx, 2);
 				return;
 			}

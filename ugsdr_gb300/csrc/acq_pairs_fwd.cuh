@@ -6,8 +6,10 @@
 // by constants), pass 1 applies the inter-step twiddle and stores; one tile,
 // two barriers per item.  fwd_rows_pair_kernel: pass 0 reads its rows from
 // global memory, pass 1 writes the spectrum over them (the part the inverse
-// gather reads).  A CTA takes up to kPairItems (Doppler, block) items of its
-// columns or rows, so that its tables and twiddle seeds are built once.
+// gather reads).  A CTA takes up to four (Doppler, block) items of its columns
+// or rows, so that its tables and twiddle seeds are built once; fewer when the
+// items are too few to fill the SMs (36 items of 50,000 points: 128 -> 121 us a
+// search).
 // Bound: issue and the latency of the loads.
 #pragma once
 
@@ -15,22 +17,27 @@
 
 namespace ugsdr_gpu {
 
-	constexpr int kPairItems = 4;
-
 	// launches, one file per kernel (acq_pairs_fwd_*.cu)
-	void launch_fwd_cols_pair_cf32(const BatchedParams& p, int items, cudaStream_t stream);
-	void launch_fwd_cols_pair_ci8(const BatchedParams& p, int items, cudaStream_t stream);
-	void launch_fwd_cols_pair_ci16(const BatchedParams& p, int items, cudaStream_t stream);
-	void launch_fwd_cols_pair_ri8(const BatchedParams& p, int items, cudaStream_t stream);
-	void launch_fwd_rows_pair(const BatchedParams& p, int items, cudaStream_t stream);
+	void launch_fwd_cols_pair_cf32(const BatchedParams& p, int items, int sm_count, cudaStream_t stream);
+	void launch_fwd_cols_pair_ci8(const BatchedParams& p, int items, int sm_count, cudaStream_t stream);
+	void launch_fwd_cols_pair_ci16(const BatchedParams& p, int items, int sm_count, cudaStream_t stream);
+	void launch_fwd_cols_pair_ri8(const BatchedParams& p, int items, int sm_count, cudaStream_t stream);
+	void launch_fwd_rows_pair(const BatchedParams& p, int items, int sm_count, cudaStream_t stream);
+
+	// items per CTA: four, or as many as leave every SM eight CTAs
+	inline int pair_items(int items, int parts, int sm_count) {
+		const long long ctas = static_cast<long long>(items) * parts;
+		return static_cast<int>(ctas >= 32LL * sm_count ? 4 : ctas >= 16LL * sm_count ? 2 : 1);
+	}
 
 	inline int pair_fwd_threads(int butterflies) {
 		return butterflies >= kPairThreads ? kPairThreads : butterflies <= 32 ? 32 : (butterflies + 31) / 32 * 32;
 	}
 
-	// grid: ceil(items / kPairItems) * ceil(N2 / 8)
+	// grid: ceil(items / per) * ceil(N2 / 8)
 	template <int ST>
-	__global__ void __launch_bounds__(kPairThreads, 2) fwd_cols_pair_kernel(const __grid_constant__ BatchedParams p, int items) {
+	__global__ void __launch_bounds__(kPairThreads, 2) fwd_cols_pair_kernel(const __grid_constant__ BatchedParams p, int items,
+		int per) {
 		extern __shared__ __align__(16) unsigned char raw[];
 		__shared__ float lut[80];
 		constexpr int CW = 8;
@@ -57,8 +64,8 @@ namespace ugsdr_gpu {
 			seeds[e] = tw_n((static_cast<uint32_t>(j) * static_cast<uint32_t>(c0 + c)) % n, n, inv_n2, false);
 		}
 		__syncthreads();
-		const int it1 = min(items, (group + 1) * kPairItems);
-		for (int item = group * kPairItems; item < it1; ++item) {
+		const int it1 = min(items, (group + 1) * per);
+		for (int item = group * per; item < it1; ++item) {
 			const int d = item / q.k_blocks;
 			const int blk = item - d * q.k_blocks;
 			const uint32_t adder = q.adders[q.d_base + d], fe_adder = q.fe_adder;
@@ -135,18 +142,20 @@ namespace ugsdr_gpu {
 	}
 
 	template <int ST>
-	void launch_fwd_cols_pair(const BatchedParams& p, int items, cudaStream_t stream) {
+	void launch_fwd_cols_pair(const BatchedParams& p, int items, int sm_count, cudaStream_t stream) {
 		const PairCols lay(p.pair.a0, p.pair.a1, 8);
 		const int seeds = lay.acc_at + static_cast<int>(sizeof(float2)) * 8 * (p.pair.a0 + 1);
-		const int grid = (items + kPairItems - 1) / kPairItems * ((p.n2 + 7) / 8);
+		const int parts = (p.n2 + 7) / 8, per = pair_items(items, parts, sm_count);
+		const int grid = (items + per - 1) / per * parts;
 		cudaFuncSetAttribute(fwd_cols_pair_kernel<ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem);
-		fwd_cols_pair_kernel<ST><<<grid, pair_fwd_threads(8 * min(p.pair.a0, p.pair.a1)), seeds, stream>>>(p, items);
+		fwd_cols_pair_kernel<ST><<<grid, pair_fwd_threads(8 * min(p.pair.a0, p.pair.a1)), seeds, stream>>>(p, items, per);
 	}
 
-	// grid: ceil(items / kPairItems) * ceil(N1 / rw); spectra elements k2 <
+	// grid: ceil(items / per) * ceil(N1 / rw); spectra elements k2 <
 	// row_keep (0: all) of each row stored
 	template <class = void>
-	__global__ void __launch_bounds__(kPairThreads, 2) fwd_rows_pair_kernel(const __grid_constant__ BatchedParams p, int items) {
+	__global__ void __launch_bounds__(kPairThreads, 2) fwd_rows_pair_kernel(const __grid_constant__ BatchedParams p, int items,
+		int per) {
 		extern __shared__ __align__(16) unsigned char raw[];
 		const int b0 = p.pair.b0, b1 = p.pair.b1, n1 = p.n1, n2 = p.n2;
 		const PairRows lay(b0, b1, p.pair.rw, 0);
@@ -163,8 +172,8 @@ namespace ugsdr_gpu {
 		__syncthreads();
 		const int keep = p.row_keep > 0 ? p.row_keep : n2;
 		const float inv_b1 = 1.0f / static_cast<float>(b1), inv_b0 = 1.0f / static_cast<float>(b0);
-		const int it1 = min(items, (group + 1) * kPairItems);
-		for (int item = group * kPairItems; item < it1; ++item) {
+		const int it1 = min(items, (group + 1) * per);
+		for (int item = group * per; item < it1; ++item) {
 			float2* rows = p.out + static_cast<size_t>(item) * p.base.n + static_cast<size_t>(r0) * n2;
 			with_radix<32>(b0, [&](auto rc) {
 				constexpr int R = decltype(rc)::value;

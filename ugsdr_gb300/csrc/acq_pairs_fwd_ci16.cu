@@ -2,7 +2,7 @@
 #include "acq_pairs_fwd.cuh"
 
 namespace ugsdr_gpu {
-	void launch_fwd_cols_pair_ci16(const BatchedParams& p, int items, cudaStream_t stream) {
-		launch_fwd_cols_pair<UGSDR_SAMPLES_CI16>(p, items, stream);
+	void launch_fwd_cols_pair_ci16(const BatchedParams& p, int items, int sm_count, cudaStream_t stream) {
+		launch_fwd_cols_pair<UGSDR_SAMPLES_CI16>(p, items, sm_count, stream);
 	}
 }

@@ -2,7 +2,7 @@
 #include "acq_pairs_fwd.cuh"
 
 namespace ugsdr_gpu {
-	void launch_fwd_cols_pair_ri8(const BatchedParams& p, int items, cudaStream_t stream) {
-		launch_fwd_cols_pair<UGSDR_SAMPLES_RI8>(p, items, stream);
+	void launch_fwd_cols_pair_ri8(const BatchedParams& p, int items, int sm_count, cudaStream_t stream) {
+		launch_fwd_cols_pair<UGSDR_SAMPLES_RI8>(p, items, sm_count, stream);
 	}
 }

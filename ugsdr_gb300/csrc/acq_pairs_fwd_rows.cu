@@ -2,12 +2,13 @@
 #include "acq_pairs_fwd.cuh"
 
 namespace ugsdr_gpu {
-	void launch_fwd_rows_pair(const BatchedParams& p, int items, cudaStream_t stream) {
+	void launch_fwd_rows_pair(const BatchedParams& p, int items, int sm_count, cudaStream_t stream) {
 		const PairSplit& s = p.pair;
 		const PairRows lay(s.b0, s.b1, s.rw, 0);
 		const int smem = lay.cs_at + static_cast<int>(sizeof(float2)) * lay.tws * s.b0;
-		const int grid = (items + kPairItems - 1) / kPairItems * ((p.n1 + s.rw - 1) / s.rw);
+		const int parts = (p.n1 + s.rw - 1) / s.rw, per = pair_items(items, parts, sm_count);
+		const int grid = (items + per - 1) / per * parts;
 		cudaFuncSetAttribute(fwd_rows_pair_kernel<>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem);
-		fwd_rows_pair_kernel<><<<grid, pair_fwd_threads(s.rw * min(s.b0, s.b1)), smem, stream>>>(p, items);
+		fwd_rows_pair_kernel<><<<grid, pair_fwd_threads(s.rw * min(s.b0, s.b1)), smem, stream>>>(p, items, per);
 	}
 }

@@ -28,6 +28,7 @@
 namespace ugsdr_gpu {
 	namespace {
 		constexpr int kTrackThreads = 256;
+		constexpr int kWindowThreads = kTrackThreads - 3 * 32;  // warps 3.. copy an epoch's first window
 		constexpr int kWinChunk = 4096;   // samples per chunk at most (a multiple of 4 x kTrackThreads)
 		constexpr int kWinPad = 128;      // window margin: taps within +-kWinPad samples of the prompt
 		constexpr int kWinFloats = kWinChunk + 2 * kWinPad + 8;  // one window: margins + 16-byte rounding
@@ -98,15 +99,38 @@ namespace ugsdr_gpu {
 			return static_cast<unsigned long long>(v);
 		}
 
-		// Loop state of one channel, held in registers of warp 0's lane 0 for the
-		// whole launch (loaded from / stored back to TrackState).
-		struct LoopState {
-			double code_phase, carrier_freq, carrier_phase_error, code_nco, code_error, code_freq;
-			float prev_re, prev_im;
-			unsigned long long phase_fx;
-			long long epoch;
-			double phase_rad;
-		};
+		// Named barriers of the loop update: one warp arrives, the others wait.
+		// Every participant reaches them once per epoch.
+		__device__ __forceinline__ void bar_arrive(int id, int threads) { asm volatile("bar.arrive %0, %1;\n" ::"r"(id), "r"(threads) : "memory"); }
+		__device__ __forceinline__ void bar_wait(int id, int threads) { asm volatile("bar.sync %0, %1;\n" ::"r"(id), "r"(threads) : "memory"); }
+		constexpr int kBarFll = 1;     // warp 2 (FLL discriminator) -> warp 0
+		constexpr int kBarWindow = 2;  // warp 1 (tap set-up) -> warps 3.. (window copy)
+
+		// Sums of each of 20 values over the warp, value *k of this lane returned:
+		// the tree of v += shfl_down(v, 16), 8, 4, 2, 1 (sums of the same pairs),
+		// each level halving the values a lane carries instead of leaving half
+		// the lanes' sums unused: 21 shuffles instead of 100.
+		__device__ __forceinline__ float reduce_scatter20(float (&v)[20], int lane, int* k) {
+			const bool b4 = lane & 16, b3 = lane & 8, b2 = lane & 4, b1 = lane & 2, b0 = lane & 1;
+			auto swap_add = [](float& keep, float other, bool hi, int o) {
+				const float mine = hi ? other : keep, sent = hi ? keep : other;
+				keep = mine + __shfl_xor_sync(0xffffffffu, sent, o);
+			};
+#pragma unroll
+			for (int i = 0; i < 10; ++i)
+				swap_add(v[i], v[i + 10], b4, 16);
+#pragma unroll
+			for (int i = 0; i < 5; ++i)
+				swap_add(v[i], v[i + 5], b3, 8);
+			swap_add(v[0], v[3], b2, 4);
+			swap_add(v[1], v[4], b2, 4);
+			v[2] += __shfl_xor_sync(0xffffffffu, v[2], 4);
+			swap_add(v[0], v[2], b1, 2);
+			v[1] += __shfl_xor_sync(0xffffffffu, v[1], 2);
+			swap_add(v[0], v[1], b0, 1);
+			*k = (b0 ? 1 + 3 * b2 : b1 ? 2 : 3 * b2) + 5 * b3 + 10 * b4;
+			return v[0];
+		}
 
 		// q - floor(q / m) m for q >= 0 and integer m, by a reciprocal and an
 		// exact correction: equals fmod(q, m).
@@ -140,9 +164,9 @@ namespace ugsdr_gpu {
 			extern __shared__ __align__(16) unsigned char s_dyn[];  // 2 windows, then (STAGED) 2 stage buffers
 			float* const s_win = reinterpret_cast<float*>(s_dyn);
 			unsigned char* const s_stage = s_dyn + 2 * kWinFloats * sizeof(float);
-			__shared__ float s_lut[80];
+			__shared__ float2 s_lut[64];  // {cos, sin} of each NCO index
 			__shared__ float s_red[kTrackThreads / 32][20];
-			__shared__ float s_sum[20];
+			__shared__ float s_ferr;
 			__shared__ unsigned long long s_holder0, s_adder;
 			__shared__ int s_mix;
 			__shared__ int s_first_len[5], s_off[5], s_split_lo, s_split_hi;
@@ -151,8 +175,8 @@ namespace ugsdr_gpu {
 
 			TrackState* st = p.states + blockIdx.x;
 			const float* rep = p.replicas + st->rep;
-			for (int i = threadIdx.x; i < 80; i += blockDim.x)
-				s_lut[i] = p.lut[i];
+			for (int i = threadIdx.x; i < 64; i += blockDim.x)
+				s_lut[i] = c2(p.lut[i + 16], p.lut[i]);
 
 			const int spm = static_cast<int>(p.spm);
 			const int period_ms = st->period_ms;
@@ -170,17 +194,19 @@ namespace ugsdr_gpu {
 			// epoch % period_ms of the next tap set-up, advanced by one per epoch
 			// (no 64-bit modulo on the serial path)
 			int ep_mod = static_cast<int>(st->epoch % period_ms);
-			const bool warp0 = threadIdx.x < 32;
+			const int warp = threadIdx.x >> 5;
 
-			LoopState ls{};
-			if (threadIdx.x == 0)
-				ls = LoopState{st->code_phase, st->carrier_freq, st->carrier_phase_error, st->code_nco, st->code_error,
-					st->code_freq, static_cast<float>(st->prev_re), static_cast<float>(st->prev_im), st->phase_fx, st->epoch,
-					st->phase_rad};
+			// The loop state lives in registers for the whole launch, each part
+			// with the warp that updates it: carrier loop in warp 0's lane 0, code
+			// loop in warp 1's, the previous prompt in warp 2's.
+			double carrier_freq = st->carrier_freq, carrier_phase_error = st->carrier_phase_error, phase_rad = st->phase_rad;
+			unsigned long long phase_fx = st->phase_fx;
+			double code_phase = st->code_phase, code_nco = st->code_nco, code_error = st->code_error, code_freq = st->code_freq;
+			float prev_re = static_cast<float>(st->prev_re), prev_im = static_cast<float>(st->prev_im);
 
-			// carrier NCO of GetEpl's Translate(signal, fs, -f, -phase), lane 0
+			// carrier NCO of GetEpl's Translate(signal, fs, -f, -phase), warp 0's lane 0
 			auto nco_setup = [&](bool first) {
-				double f = -ls.carrier_freq;
+				double f = -carrier_freq;
 				s_mix = fabs(f) != 0.0;
 				if (f < 0)
 					f = p.fs + f;
@@ -189,7 +215,7 @@ namespace ugsdr_gpu {
 					// reduced to [0, 2 pi), 32-bit holder and adder; carried in the
 					// upper half of the 64-bit accumulator, whose top 6 bits are then
 					// the 32-bit NCO's index and whose wrap is its wrap
-					double ph = fmod(-ls.phase_rad, 2 * kPi);
+					double ph = fmod(-phase_rad, 2 * kPi);
 					if (ph < 0)
 						ph = __dadd_rn(ph, 2 * kPi);
 					const unsigned long long a32 = static_cast<unsigned long long>(__ddiv_rn(__dmul_rn(4294967296.0, f), p.fs));
@@ -209,16 +235,16 @@ namespace ugsdr_gpu {
 				if (av >= kTwo64)
 					av = 0.0;
 				s_adder = static_cast<unsigned long long>(av);
-				s_holder0 = 0ull - ls.phase_fx;
+				s_holder0 = 0ull - phase_fx;
 			};
 			// CorrelateSplit set-up of the five taps from the code phase, lanes 0-4
-			// of warp 0 (one tap each): split point, weight, replica offset.
+			// of warp 1 (one tap each): split point, weight, replica offset.
 			auto tap_setup = [&]() {
-				const double code_phase = __shfl_sync(0xffffffffu, ls.code_phase, 0);
+				const double cp = __shfl_sync(0xffffffffu, code_phase, 0);
 				long long fp = 0;
 				int fl = 0;
 				if (lane < 5) {
-					const double ph = code_phase - fs_ms * static_cast<double>(ep_mod);
+					const double ph = cp - fs_ms * static_cast<double>(ep_mod);
 					double q = ph + spc * p.offsets[lane];
 					while (q < 0)
 						q += period;
@@ -254,14 +280,14 @@ namespace ugsdr_gpu {
 				}
 			};
 			// chunk k's window (n_c + 2 kWinPad entries from table index x0) into
-			// window buf: 16-byte copies from x0 rounded down to 4 entries (the
-			// table is padded for the rounded-up end)
-			auto fetch_window = [&](int buf, long long x0, int n_c) {
+			// window buf by `threads` threads, this one number t: 16-byte copies from
+			// x0 rounded down to 4 entries (the table is padded for the rounded-up end)
+			auto fetch_window = [&](int buf, long long x0, int n_c, int t, int threads) {
 				const long long a0 = x0 & ~3ll;
 				const int n_copy = (static_cast<int>(x0 - a0) + n_c + 2 * kWinPad + 3) & ~3;
 				float* dst = s_win + buf * kWinFloats;
 				const float* src = rep + a0;
-				for (int o = 4 * threadIdx.x; o < n_copy; o += 4 * blockDim.x)
+				for (int o = 4 * t; o < n_copy; o += 4 * threads)
 					cp_async_g<16>(dst + o, src + o);
 			};
 			// samples of global chunk gi = epoch * n_chunks + chunk into stage buffer gi & 1
@@ -285,15 +311,14 @@ namespace ugsdr_gpu {
 						cp_async_g<4>(dst + o, src + o);
 				}
 			};
-			if (warp0) {
-				if (lane == 0)
-					nco_setup(ls.epoch == 0);  // the channel's first epoch (not every launch: runs split differently agree)
+			if (warp == 0 && lane == 0)
+				nco_setup(st->epoch == 0);  // the channel's first epoch (not every launch: runs split differently agree)
+			if (warp == 1)
 				tap_setup();
-			}
 			if constexpr (STAGED)
 				stage(0);
 			__syncthreads();  // s_wstart of epoch 0
-			fetch_window(0, s_wstart, min(CH, spm));
+			fetch_window(0, s_wstart, min(CH, spm), threadIdx.x, kTrackThreads);
 			cp_async_commit();
 
 			for (int ep = 0; ep < p.n_epochs; ++ep) {
@@ -303,10 +328,15 @@ namespace ugsdr_gpu {
 					off[t] = s_off[t];
 				const long long wstart = s_wstart;
 				const int split_lo = s_split_lo, split_hi = s_split_hi;
-				float acc[20];
+				// per side (left, right of the split) I and Q sums of the taps: taps
+				// 0-3 as two packed pairs (one packed multiply-add for two taps), tap 4
+				float2 acc_i[2][2], acc_q[2][2];
+				float acc_4i[2], acc_4q[2];
 #pragma unroll
-				for (int k = 0; k < 20; ++k)
-					acc[k] = 0.f;
+				for (int k = 0; k < 2; ++k) {
+					acc_i[k][0] = acc_i[k][1] = acc_q[k][0] = acc_q[k][1] = c2(0.f, 0.f);
+					acc_4i[k] = acc_4q[k] = 0.f;
+				}
 				const unsigned long long adder = s_adder;
 				unsigned long long holder = s_holder0 + static_cast<unsigned long long>(threadIdx.x) * adder;
 				const unsigned long long hstep = static_cast<unsigned long long>(blockDim.x) * adder;
@@ -319,7 +349,7 @@ namespace ugsdr_gpu {
 					cp_async_wait_all();  // this chunk's window and samples (issued one chunk earlier)
 					__syncthreads();      // ... for every thread; the other buffers were last read by chunk gi - 1
 					if (k + 1 < n_chunks) {
-						fetch_window((gi + 1) & 1, wstart + c0 + CH, min(CH, spm - c0 - CH));
+						fetch_window((gi + 1) & 1, wstart + c0 + CH, min(CH, spm - c0 - CH), threadIdx.x, kTrackThreads);
 						if constexpr (STAGED)
 							stage(gi + 1);
 						cp_async_commit();
@@ -353,25 +383,40 @@ namespace ugsdr_gpu {
 								break;
 							float2 x = xs[u];
 							if (mix) {
-								const uint32_t idx = static_cast<uint32_t>(holder >> 58);
-								const float c = s_lut[idx + 16], s = s_lut[idx];
-								x = c2(__fsub_rn(__fmul_rn(x.x, c), __fmul_rn(x.y, s)), __fadd_rn(__fmul_rn(x.x, s), __fmul_rn(x.y, c)));
+								const float2 w = s_lut[static_cast<uint32_t>(holder >> 58)];
+								x = c2(__fsub_rn(__fmul_rn(x.x, w.x), __fmul_rn(x.y, w.y)), __fadd_rn(__fmul_rn(x.x, w.y), __fmul_rn(x.y, w.x)));
 							}
 							holder += hstep;
+							float cv[5];
 #pragma unroll
-							for (int t = 0; t < 5; ++t) {
-								const float cv = win[i + off[t]];
-								// the two CorrelateSplit partial sums
-								bool left = MODE == kLeft;
-								if constexpr (MODE == kMixed)
-									left = c0 + i < s_first_len[t];
-								if (left) {
-									acc[4 * t] += x.x * cv;
-									acc[4 * t + 1] += x.y * cv;
+							for (int t = 0; t < 5; ++t)
+								cv[t] = win[i + off[t]];
+							if constexpr (MODE != kMixed) {
+								// all taps on one side: two taps per packed multiply-add
+								// (each half rounds as the single one; the products are exact)
+#pragma unroll
+								for (int h = 0; h < 2; ++h) {
+									const float2 c = c2(cv[2 * h], cv[2 * h + 1]);
+									acc_i[MODE][h] = __ffma2_rn(c2(x.x, x.x), c, acc_i[MODE][h]);
+									acc_q[MODE][h] = __ffma2_rn(c2(x.y, x.y), c, acc_q[MODE][h]);
 								}
-								else {
-									acc[4 * t + 2] += x.x * cv;
-									acc[4 * t + 3] += x.y * cv;
+								acc_4i[MODE] = fmaf(x.x, cv[4], acc_4i[MODE]);
+								acc_4q[MODE] = fmaf(x.y, cv[4], acc_4q[MODE]);
+							}
+							else {
+								// the two CorrelateSplit partial sums, tap by tap
+#pragma unroll
+								for (int t = 0; t < 5; ++t) {
+									const bool left = c0 + i < s_first_len[t];
+#pragma unroll
+									for (int k = 0; k < 2; ++k) {
+										float& ai = t == 4 ? acc_4i[k] : t & 1 ? acc_i[k][(t & 3) >> 1].y : acc_i[k][(t & 3) >> 1].x;
+										float& aq = t == 4 ? acc_4q[k] : t & 1 ? acc_q[k][(t & 3) >> 1].y : acc_q[k][(t & 3) >> 1].x;
+										if (left == (k == 0)) {
+											ai = fmaf(x.x, cv[t], ai);
+											aq = fmaf(x.y, cv[t], aq);
+										}
+									}
 								}
 							}
 						}
@@ -386,144 +431,162 @@ namespace ugsdr_gpu {
 							correlate4(i0, std::integral_constant<int, kMixed>{});
 					}
 				}
-				// block reduction of the 20 partial sums
+				// warp sums of the 20 partial sums (value 4 t + 2 side + {I, Q})
+				{
+					float v[20];
 #pragma unroll
-				for (int k = 0; k < 20; ++k) {
-					float v = acc[k];
+					for (int k = 0; k < 2; ++k) {
 #pragma unroll
-					for (int o = 16; o > 0; o >>= 1)
-						v += __shfl_down_sync(0xffffffffu, v, o);
-					if (lane == 0)
-						s_red[threadIdx.x >> 5][k] = v;
+						for (int h = 0; h < 2; ++h) {
+							v[8 * h + 2 * k] = acc_i[k][h].x;
+							v[8 * h + 2 * k + 1] = acc_q[k][h].x;
+							v[8 * h + 4 + 2 * k] = acc_i[k][h].y;
+							v[8 * h + 4 + 2 * k + 1] = acc_q[k][h].y;
+						}
+						v[16 + 2 * k] = acc_4i[k];
+						v[16 + 2 * k + 1] = acc_4q[k];
+					}
+					int k;
+					const float sum = reduce_scatter20(v, lane, &k);
+					s_red[warp][k] = sum;
 				}
+				const int my_tap = lane < 5 ? lane : 0;
+				const double rel = s_rel[my_tap];  // before warp 1 sets up the next epoch's
 				__syncthreads();
-				if (warp0) {
-					if (lane < 20) {
-						float v = 0.f;
+				// Loop update, its independent parts on warps of their own: 0 the
+				// carrier loop and NCO, 1 the code loop and tap set-up, 2 the FLL
+				// discriminator, 3 the output's taps; the others copy the next
+				// epoch's first window as soon as warp 1 has placed it.  Warps 0-3
+				// each form the taps (lanes 0-4) from the warp sums.
+				const bool more = ep + 1 < p.n_epochs;
+				TrackOut* const out = p.out ? p.out + static_cast<size_t>(ep) * p.n_channels + blockIdx.x : nullptr;
+				float tap_re = 0.f, tap_im = 0.f;
+				if (warp < 4) {
+					float v = 0.f;
+					if (lane < 20)
 						for (int w = 0; w < kTrackThreads / 32; ++w)
 							v += s_red[w][lane];
-						s_sum[lane] = v;
-					}
-					__syncwarp();
-					// AddWithPhase per tap (lanes 0-4): the reference's comparison
+					// AddWithPhase per tap: the reference's comparison
 					// |l / rel + r / (1 - rel)| > |l / rel| multiplied through by
 					// rel (1 - rel) > 0; taps rounded to float as the reference's
-					float tap_re = 0.f, tap_im = 0.f;
-					if (lane < 5) {
-						float lr = s_sum[4 * lane], li = s_sum[4 * lane + 1], rr = s_sum[4 * lane + 2], ri = s_sum[4 * lane + 3];
-						const double rel = s_rel[lane];
-						if (rel < 0.5) {
-							float t0 = lr; lr = rr; rr = t0;
-							t0 = li; li = ri; ri = t0;
-						}
-						const double a = static_cast<double>(lr) * (1.0 - rel);
-						const bool plus = fabs(a + static_cast<double>(rr) * rel) > fabs(a);
-						// lhs +- rhs of complex<float>: float sums, as the reference adds
-						tap_re = plus ? __fadd_rn(lr, rr) : __fsub_rn(lr, rr);
-						tap_im = plus ? __fadd_rn(li, ri) : __fsub_rn(li, ri);
+					float lr = __shfl_sync(0xffffffffu, v, 4 * my_tap), li = __shfl_sync(0xffffffffu, v, 4 * my_tap + 1);
+					float rr = __shfl_sync(0xffffffffu, v, 4 * my_tap + 2), ri = __shfl_sync(0xffffffffu, v, 4 * my_tap + 3);
+					if (rel < 0.5) {
+						float t0 = lr; lr = rr; rr = t0;
+						t0 = li; li = ri; ri = t0;
 					}
-					float taps_re[5], taps_im[5];
-#pragma unroll
-					for (int t = 0; t < 5; ++t) {
-						taps_re[t] = __shfl_sync(0xffffffffu, tap_re, t);
-						taps_im[t] = __shfl_sync(0xffffffffu, tap_im, t);
-					}
-					const float pr = taps_re[2], pi = taps_im[2];
-					const float ppr = __shfl_sync(0xffffffffu, ls.prev_re, 0), ppi = __shfl_sync(0xffffffffu, ls.prev_im, 0);
-					// discriminators in the reference's float types, side by side:
-					// lane 0 PLL atan(imag / real), 1 FLL atan2(cross, dot), 2 |E|, 3 |L|
-					float part = 0.f;
-					double part_d = 0.0;  // nco_mode 1: the reference's double atan of the float ratio
+					const double a = static_cast<double>(lr) * (1.0 - rel);
+					const bool plus = fabs(a + static_cast<double>(rr) * rel) > fabs(a);
+					// lhs +- rhs of complex<float>: float sums, as the reference adds
+					tap_re = plus ? __fadd_rn(lr, rr) : __fsub_rn(lr, rr);
+					tap_im = plus ? __fadd_rn(li, ri) : __fsub_rn(li, ri);
+				}
+				if (warp == 0) {
+					const float pr = __shfl_sync(0xffffffffu, tap_re, 2), pi = __shfl_sync(0xffffffffu, tap_im, 2);
+					// PLL discriminator atan(imag / real): float, or (nco_mode 1) the
+					// reference's double atan of the float ratio; the reference divides
+					// by 2 pi, the 64-bit NCO mode multiplies by the reciprocal
+					double err = 0.0;
 					if (lane == 0) {
 						if (p.nco_mode == 1)
-							part_d = pr != 0.f ? atan(static_cast<double>(__fdiv_rn(pi, pr))) : 0.0;
+							err = (pr != 0.f ? atan(static_cast<double>(__fdiv_rn(pi, pr))) : 0.0) / (kPi * 2.0);
 						else
-							part = pr != 0.f ? atanf(__fdiv_rn(pi, pr)) : 0.f;
-					}
-					else if (lane == 1) {
-						const float cross = __fsub_rn(__fmul_rn(pr, ppi), __fmul_rn(ppr, pi));
-						const float dot = fabsf(__fadd_rn(__fmul_rn(pr, ppr), __fmul_rn(ppi, pi)));
-						part = atan2f(cross, dot);
-					}
-					else if (lane == 2) {
-						part = hypotf(taps_re[1], taps_im[1]);
-					}
-					else if (lane == 3) {
-						part = hypotf(taps_re[3], taps_im[3]);
-					}
-					const float ferr_f = __shfl_sync(0xffffffffu, part, 1);
-					const float ea = __shfl_sync(0xffffffffu, part, 2);
-					const float la = __shfl_sync(0xffffffffu, part, 3);
-					if (lane == 0) {
-						// the reference divides by 2 pi and pi (nco_mode 1 keeps the
-						// quotients); the 64-bit NCO mode multiplies by the reciprocals
-						const double err = p.nco_mode == 1 ? part_d / (kPi * 2.0) : static_cast<double>(part) * (0.5 / kPi);
-						const double ferr = p.nco_mode == 1 ? static_cast<double>(ferr_f) / kPi : static_cast<double>(ferr_f) * (1.0 / kPi);
+							err = static_cast<double>(pr != 0.f ? atanf(__fdiv_rn(pi, pr)) : 0.f) * (0.5 / kPi);
 						// UpdatePhase (tracking_parameters.hpp:163-165) with the pre-update frequency
-						ls.phase_fx += frac_to_fx(ls.carrier_freq * 1e-3);
+						phase_fx += frac_to_fx(carrier_freq * 1e-3);
 						if (p.nco_mode == 1)  // the radian phase: the reference NCO mode's carrier phase
-							ls.phase_rad = __dadd_rn(ls.phase_rad, __ddiv_rn(__dmul_rn(2 * kPi, ls.carrier_freq), 1000.0));
+							phase_rad = __dadd_rn(phase_rad, __ddiv_rn(__dmul_rn(2 * kPi, carrier_freq), 1000.0));
+						phase_fx += static_cast<unsigned long long>(llrint(err * (kTwo64 / 4.0)));
+					}
+					bar_wait(kBarFll, 64);
+					if (lane == 0) {
+						const float ferr_f = s_ferr;
+						const double ferr = p.nco_mode == 1 ? static_cast<double>(ferr_f) / kPi : static_cast<double>(ferr_f) * (1.0 / kPi);
 						// Pll(prompt) (tracking_parameters.hpp:495-511), loop filter in FP64
 						// in the reference's operation order, nothing contracted
-						ls.carrier_freq = __dadd_rn(ls.carrier_freq, __dsub_rn(__dsub_rn(__dmul_rn(p.k1_pll, err),
-							__dmul_rn(p.k2_pll, ls.carrier_phase_error)), __dmul_rn(p.k3_pll, ferr)));
-						ls.carrier_phase_error = err;
-						ls.phase_fx += static_cast<unsigned long long>(llrint(err * (kTwo64 / 4.0)));
+						carrier_freq = __dadd_rn(carrier_freq, __dsub_rn(__dsub_rn(__dmul_rn(p.k1_pll, err),
+							__dmul_rn(p.k2_pll, carrier_phase_error)), __dmul_rn(p.k3_pll, ferr)));
+						carrier_phase_error = err;
 						if (p.nco_mode == 1)
-							ls.phase_rad = __dadd_rn(ls.phase_rad, __ddiv_rn(__dmul_rn(err, kPi), 2.0));
-						ls.prev_re = pr;
-						ls.prev_im = pi;
+							phase_rad = __dadd_rn(phase_rad, __ddiv_rn(__dmul_rn(err, kPi), 2.0));
+						nco_setup(false);
+					}
+				}
+				else if (warp == 1) {
+					const float mag = hypotf(tap_re, tap_im);
+					const float ea = __shfl_sync(0xffffffffu, mag, 1), la = __shfl_sync(0xffffffffu, mag, 3);
+					if (lane == 0) {
 						// Dll(early, late) (tracking_parameters.hpp:513-528)
 						double ce = 0.0;
 						if (ea + la != 0.f)
 							ce = __fdiv_rn(__fsub_rn(ea, la), __fadd_rn(ea, la));
-						ls.code_nco = __dadd_rn(ls.code_nco, __dmul_rn(__dadd_rn(__dmul_rn(p.k1_dll, __dsub_rn(ce, ls.code_error)),
+						code_nco = __dadd_rn(code_nco, __dmul_rn(__dadd_rn(__dmul_rn(p.k1_dll, __dsub_rn(ce, code_error)),
 							__dmul_rn(p.k2_dll, ce)), dll_scale));
-						ls.code_error = ce;
-						ls.code_freq = __dsub_rn(base_freq, ls.code_nco);
+						code_error = ce;
+						code_freq = __dsub_rn(base_freq, code_nco);
 						// code_freq / base as the reference divides it (nco_mode 1), by the
 						// reciprocal otherwise (one FP64 division less on the epoch's serial path)
-						const double ratio = p.nco_mode == 1 ? __ddiv_rn(ls.code_freq, base_freq) : __dmul_rn(ls.code_freq, inv_base);
-						ls.code_phase = __dsub_rn(ls.code_phase, __dmul_rn(half_fs_ms, __dsub_rn(ratio, 1.0)));
-						if (p.out) {
-							TrackOut o;
-							for (int t = 0; t < 5; ++t) {
-								o.taps[t][0] = taps_re[t];
-								o.taps[t][1] = taps_im[t];
-							}
-							o.carrier_frequency = ls.carrier_freq;
-							o.carrier_phase = p.nco_mode == 1 ? ls.phase_rad : static_cast<double>(ls.phase_fx) / kTwo64 * 2 * kPi;
-							o.code_phase = ls.code_phase;
-							o.code_frequency = ls.code_freq;
-							o.phase_error = err;
-							o.code_error = ce;
-							p.out[static_cast<size_t>(ep) * p.n_channels + blockIdx.x] = o;
-						}
-						++ls.epoch;
-						nco_setup(false);
+						const double ratio = p.nco_mode == 1 ? __ddiv_rn(code_freq, base_freq) : __dmul_rn(code_freq, inv_base);
+						code_phase = __dsub_rn(code_phase, __dmul_rn(half_fs_ms, __dsub_rn(ratio, 1.0)));
 					}
 					__syncwarp();
 					ep_mod = ep_mod + 1 == period_ms ? 0 : ep_mod + 1;
-					if (ep + 1 < p.n_epochs)
+					if (more)
 						tap_setup();
+					bar_arrive(kBarWindow, kWindowThreads + 32);
+				}
+				else if (warp == 2) {
+					const float pr = __shfl_sync(0xffffffffu, tap_re, 2), pi = __shfl_sync(0xffffffffu, tap_im, 2);
+					if (lane == 0) {
+						// FLL discriminator atan2(cross, dot) in the reference's float types
+						const float cross = __fsub_rn(__fmul_rn(pr, prev_im), __fmul_rn(prev_re, pi));
+						const float dot = fabsf(__fadd_rn(__fmul_rn(pr, prev_re), __fmul_rn(pi, prev_im)));
+						s_ferr = atan2f(cross, dot);
+						prev_re = pr;
+						prev_im = pi;
+					}
+					__syncwarp();
+					bar_arrive(kBarFll, 64);
+				}
+				else {
+					if (warp == 3 && lane < 5 && out) {
+						out->taps[lane][0] = tap_re;
+						out->taps[lane][1] = tap_im;
+					}
+					bar_wait(kBarWindow, kWindowThreads + 32);
+					if (more) {
+						fetch_window(((ep + 1) * n_chunks) & 1, s_wstart, min(CH, spm), threadIdx.x - (kTrackThreads - kWindowThreads),
+							kWindowThreads);
+						cp_async_commit();
+					}
 				}
 				__syncthreads();  // the next epoch's NCO and taps
-				if (ep + 1 < p.n_epochs) {
-					fetch_window(((ep + 1) * n_chunks) & 1, s_wstart, min(CH, spm));
-					cp_async_commit();
+				if (out && threadIdx.x == 0) {
+					out->carrier_frequency = carrier_freq;
+					out->carrier_phase = p.nco_mode == 1 ? phase_rad : static_cast<double>(phase_fx) / kTwo64 * 2 * kPi;
+					out->phase_error = carrier_phase_error;
+				}
+				if (out && threadIdx.x == 32) {
+					out->code_phase = code_phase;
+					out->code_frequency = code_freq;
+					out->code_error = code_error;
 				}
 			}
 			if (threadIdx.x == 0) {
-				st->code_phase = ls.code_phase;
-				st->carrier_freq = ls.carrier_freq;
-				st->carrier_phase_error = ls.carrier_phase_error;
-				st->code_nco = ls.code_nco;
-				st->code_error = ls.code_error;
-				st->code_freq = ls.code_freq;
-				st->prev_re = ls.prev_re;
-				st->prev_im = ls.prev_im;
-				st->phase_fx = ls.phase_fx;
-				st->epoch = ls.epoch;
+				st->carrier_freq = carrier_freq;
+				st->carrier_phase_error = carrier_phase_error;
+				st->phase_fx = phase_fx;
+				st->epoch += p.n_epochs;
+			}
+			if (threadIdx.x == 32) {
+				st->code_phase = code_phase;
+				st->code_nco = code_nco;
+				st->code_error = code_error;
+				st->code_freq = code_freq;
+			}
+			if (threadIdx.x == 64) {
+				st->prev_re = prev_re;
+				st->prev_im = prev_im;
 			}
 		}
 	}
