@@ -2,10 +2,11 @@
 // the suppression engine the digital front end runs after resampling
 // (src/dfe/dfe.hpp:199-202).
 //
-//   detect_kernel       the detector's STFT, one warp per column with the
-//                       128-point transform in registers and shuffles
-//                       (Warp128), then the eight strongest bins with their
-//                       peak / sigma (JammingDetector::IntermediateDetection,
+//   detect_kernel       the detector's STFT, eight lanes per column with the
+//                       128-point transform in registers and one exchange
+//                       through shared memory (Octet128), then one thread per
+//                       column for the eight strongest bins with their peak /
+//                       sigma (JammingDetector::IntermediateDetection,
 //                       src/antijamming/jamming_detection.hpp:113-128) and
 //                       each CTA's occupation histograms
 //   stft_kernel         the per-op STFT (spectra out): columns per CTA in
@@ -14,8 +15,8 @@
 //   jn_sum_kernel       round, then the reported J/N sums; only the detection
 //                       list goes back to the host
 //   wideband_kernel     FilterWideband (src/antijamming/jse.hpp:70-87) fused,
-//                       one warp per run of output slots: the covering columns
-//                       re-transformed from the samples (Warp128), bins with
+//                       eight lanes per run of output slots: the covering columns
+//                       re-transformed from the samples (Octet128), bins with
 //                       |.| >= 20 zeroed, inverse transforms scaled 2/W,
 //                       overlap-added in column order in registers
 //   istft_cols_kernel,  the per-op OverlapAndAdd (src/math/stft.hpp:63-75):
@@ -37,7 +38,6 @@ namespace ugsdr_gpu {
 		constexpr int kNullHalfWidth = 3;      // null_window_size (82)
 		constexpr float kJnThreshold = 6.0f;   // j_s_threshold (78)
 		constexpr double kProbability = 0.9;   // probability_threshold (79)
-		constexpr float kWidebandLevel = 20.0f;  // j_s_absolute_threshold (jse.hpp:43)
 		constexpr int kNarrowNull = 128;       // null_window_size (jse.hpp:47)
 		constexpr int kDetectWindow = 128;     // Transform's defaults (stft.hpp:19)
 		constexpr int kDetectOverlap = 96;
@@ -119,82 +119,6 @@ namespace ugsdr_gpu {
 			float2* s;             // cols x w spectra
 		};
 
-		__device__ __forceinline__ float magnitude(float2 v) { return sqrtf(v.x * v.x + v.y * v.y); }
-
-		// The warp's column, magnitudes in registers (mv[j] of lane l is bin idx[j]):
-		// kMaxCandidates rounds of first-max — the largest magnitude (redux max
-		// over the bit patterns, which order as non-negative floats do), then
-		// the lowest bin holding it (redux min), as std::max_element — each
-		// followed by nulling +-3 bins (NullRegion, jamming_detection.hpp:
-		// 101-110); then the float mean and unbiased sigma of the nulled
-		// magnitudes with SequentialMeanStdDev's formula (src/math/
-		// mean_stddev.hpp:29-42; the sums in warp-tree order) and J/N =
-		// peak / sigma.  Candidates with J/N < 6 are erased, the rest
-		// kept in order: kept candidate r of column `col` goes to [r][col] and
-		// into the CTA's round-r occupation histogram.
-		__device__ void detect_column(float (&mv)[kDetectBins / 32], const int (&idx)[kDetectBins / 32], const DetectScratch& d,
-			size_t col, size_t cols, int* s_hist, unsigned int* s_total) {
-			constexpr int J = kDetectBins / 32;
-			const int lane = threadIdx.x & 31;
-			int bins[kMaxCandidates];
-			float peaks[kMaxCandidates];
-#pragma unroll
-			for (int r = 0; r < kMaxCandidates; ++r) {
-				unsigned int top = 0;
-#pragma unroll
-				for (int j = 0; j < J; ++j)
-					top = max(top, __float_as_uint(mv[j]));
-				top = __reduce_max_sync(0xffffffffu, top);
-				unsigned int first = 0xffffffffu;
-#pragma unroll
-				for (int j = 0; j < J; ++j)
-					if (__float_as_uint(mv[j]) == top)
-						first = min(first, static_cast<unsigned int>(idx[j]));
-				const int bi = static_cast<int>(__reduce_min_sync(0xffffffffu, first));
-				bins[r] = bi;
-				peaks[r] = __uint_as_float(top);
-#pragma unroll
-				for (int j = 0; j < J; ++j) {
-					const int dist = (idx[j] - bi + kDetectBins) % kDetectBins;
-					if (dist <= kNullHalfWidth || dist >= kDetectBins - kNullHalfWidth)
-						mv[j] = 0.0f;
-				}
-			}
-			float q = 0.0f, s = 0.0f;
-#pragma unroll
-			for (int j = 0; j < J; ++j) {
-				q = __fadd_rn(q, __fmul_rn(mv[j], mv[j]));
-				s = __fadd_rn(s, mv[j]);
-			}
-			for (int o = 16; o > 0; o >>= 1) {
-				q = __fadd_rn(q, __shfl_xor_sync(0xffffffffu, q, o));
-				s = __fadd_rn(s, __shfl_xor_sync(0xffffffffu, s, o));
-			}
-			if (lane != 0)
-				return;
-			const float fw = static_cast<float>(kDetectBins);
-			const float var = __fdiv_rn(__fsub_rn(q, __fdiv_rn(__fmul_rn(s, s), fw)), static_cast<float>(kDetectBins - 1));
-			const float sigma = __fsqrt_rn(var);
-			int c = 0;
-#pragma unroll
-			for (int r = 0; r < kMaxCandidates; ++r) {
-				// double(peak) / double(sigma) < 6 exactly when peak - 6 sigma < 0
-				// (two floats' double quotient cannot round onto 6 unless it is 6),
-				// and fmaf rounds that difference once, keeping its sign: the
-				// reference's double test without FP64 (a NaN stays, as in
-				// remove_if(jn < threshold)).  The kept J/N is the float quotient.
-				if (!(fmaf(-kJnThreshold, sigma, peaks[r]) < 0.0f)) {
-					d.bins[static_cast<size_t>(c) * cols + col] = static_cast<uint8_t>(bins[r]);
-					d.jn[static_cast<size_t>(c) * cols + col] = __fdiv_rn(peaks[r], sigma);
-					atomicAdd(&s_hist[c * kDetectBins + bins[r]], 1);
-					++c;
-				}
-			}
-			for (int r = c; r < kMaxCandidates; ++r)
-				d.bins[static_cast<size_t>(r) * cols + col] = kNoBin;
-			atomicAdd(s_total, static_cast<unsigned int>(c));
-		}
-
 		template <class F>
 		__global__ void __launch_bounds__(kJamThreads) stft_kernel(StftParams p) {
 			extern __shared__ float2 sm[];
@@ -223,122 +147,230 @@ namespace ugsdr_gpu {
 			}
 		}
 
-		// 128-point DFT of one warp in registers: lane l holds v[j] =
-		// x[l + 32 j]; a radix-4 step over j, the twiddle W_128^{l k1}, then per
-		// k1 a 32-point DFT across the lanes in five radix-2
-		// decimation-in-frequency shuffle stages (h = 16 .. 1).  Lane l then
-		// holds X[k1 + 4 rev5(l)] in v[k1] (X[k1 + 4 k2] = sum_l W_128^{l k1}
-		// W_32^{l k2} sum_j x[l + 32 j] W_4^{j k1}).  The inverse runs the
-		// network backwards with conjugate twiddles, from that layout back to
-		// x[l + 32 j], unnormalised (x 128).  No shared memory, no barrier.
-		struct Warp128 {
-			float2 tw[3];  // W_128^{l k1}, k1 = 1..3
-			float2 ts[5];  // W_{2h}^{l mod h}, h = 16, 8, 4, 2, 1
-			__device__ __forceinline__ void init(const float2* tab, int lane) {
+		// 128-point DFT of one column by eight lanes, four columns per warp.  Lane
+		// l holds v[j] = x[l + 8 j]: a 16-point DFT over j in registers, the twiddle
+		// W_128^{l k1}, one exchange through shared memory, and for the lane's k1 =
+		// l and l + 8 an 8-point DFT over the lanes' values; lane l then holds
+		// X[l + 8 m] in v[m].  The inverse runs backwards with conjugate twiddles,
+		// unnormalised (x 128).  16 stores and 16 loads per lane and four columns,
+		// against the 40 two-word shuffles per column of one warp per column.
+		// Exchange tiles: element (k1, l) at 9 k1 + l, columns 152 apart, so that
+		// half-warps of stores and loads touch every bank once.
+		constexpr int kOctetTile = 152;
+		struct Octet128 {
+			float2 tw[15];   // W_128^{l k1}, k1 = 1..15
+			float2* tile;    // the column's exchange tile
+			int l;
+			__device__ __forceinline__ void init(const float2* __restrict__ table, float2* warp_tiles) {
+				const int lane = threadIdx.x & 31;
+				l = lane & 7;
+				tile = warp_tiles + (lane >> 3) * kOctetTile;
 #pragma unroll
-				for (int k1 = 1; k1 < 4; ++k1)
-					tw[k1 - 1] = tab[(lane * k1) & 127];
+				for (int k1 = 1; k1 < 16; ++k1)
+					tw[k1 - 1] = __ldg(table + l * k1);
+			}
+			__device__ __forceinline__ void forward(float2 (&v)[16]) const {
+				Dft<16, false>::run(v);
+				tile[l] = v[0];
 #pragma unroll
-				for (int st = 0; st < 5; ++st) {
-					const int h = 16 >> st;
-					ts[st] = tab[(lane & (h - 1)) * (64 / h)];
+				for (int k1 = 1; k1 < 16; ++k1)
+					tile[9 * k1 + l] = cmul(v[k1], tw[k1 - 1]);
+				__syncwarp();
+				float2 a[8], b[8];
+#pragma unroll
+				for (int i = 0; i < 8; ++i) {
+					a[i] = tile[9 * l + i];
+					b[i] = tile[9 * (l + 8) + i];
+				}
+				__syncwarp();  // the next exchange may write
+				Dft<8, false>::run(a);
+				Dft<8, false>::run(b);
+#pragma unroll
+				for (int i = 0; i < 8; ++i) {
+					v[2 * i] = a[i];
+					v[2 * i + 1] = b[i];
 				}
 			}
-			__device__ __forceinline__ static int natural(int j, int lane) { return j + 4 * static_cast<int>(__brev(lane) >> 27); }
-			__device__ __forceinline__ void forward(float2 (&v)[4], int lane) const {
-				const float2 a0 = cadd(v[0], v[2]), a1 = csub(v[0], v[2]);
-				const float2 b0 = cadd(v[1], v[3]), dd = csub(v[1], v[3]);
-				const float2 b1 = c2(dd.y, -dd.x);  // (v1 - v3)(-i)
-				v[0] = cadd(a0, b0);
-				v[2] = csub(a0, b0);
-				v[1] = cadd(a1, b1);
-				v[3] = csub(a1, b1);
+			__device__ __forceinline__ void inverse(float2 (&v)[16]) const {
+				float2 a[8], b[8];
 #pragma unroll
-				for (int k1 = 1; k1 < 4; ++k1)
-					v[k1] = cmul(v[k1], tw[k1 - 1]);
-#pragma unroll
-				for (int st = 0; st < 5; ++st) {
-					const int h = 16 >> st;
-					const bool hi = (lane & h) != 0;
-#pragma unroll
-					for (int j = 0; j < 4; ++j) {
-						const float2 o = c2(__shfl_xor_sync(0xffffffffu, v[j].x, h), __shfl_xor_sync(0xffffffffu, v[j].y, h));
-						v[j] = hi ? cmul(csub(o, v[j]), ts[st]) : cadd(v[j], o);
-					}
+				for (int i = 0; i < 8; ++i) {
+					a[i] = v[2 * i];
+					b[i] = v[2 * i + 1];
 				}
-			}
-			__device__ __forceinline__ void inverse(float2 (&v)[4], int lane) const {
+				Dft<8, true>::run(a);
+				Dft<8, true>::run(b);
 #pragma unroll
-				for (int st = 4; st >= 0; --st) {
-					const int h = 16 >> st;
-					const bool hi = (lane & h) != 0;
-#pragma unroll
-					for (int j = 0; j < 4; ++j) {
-						const float2 q = hi ? cmulc(v[j], ts[st]) : v[j];
-						const float2 o = c2(__shfl_xor_sync(0xffffffffu, q.x, h), __shfl_xor_sync(0xffffffffu, q.y, h));
-						v[j] = hi ? csub(o, q) : cadd(q, o);
-					}
+				for (int i = 0; i < 8; ++i) {
+					tile[9 * l + i] = a[i];
+					tile[9 * (l + 8) + i] = b[i];
 				}
+				__syncwarp();
+				v[0] = tile[l];
 #pragma unroll
-				for (int k1 = 1; k1 < 4; ++k1)
-					v[k1] = cmulc(v[k1], tw[k1 - 1]);
-				const float2 a0 = cadd(v[0], v[2]), a1 = csub(v[0], v[2]);
-				const float2 b0 = cadd(v[1], v[3]), dd = csub(v[1], v[3]);
-				const float2 b1 = c2(-dd.y, dd.x);  // (v1 - v3)(+i)
-				v[0] = cadd(a0, b0);
-				v[2] = csub(a0, b0);
-				v[1] = cadd(a1, b1);
-				v[3] = csub(a1, b1);
+				for (int k1 = 1; k1 < 16; ++k1)
+					v[k1] = cmulc(tile[9 * k1 + l], tw[k1 - 1]);
+				__syncwarp();
+				Dft<16, true>::run(v);
 			}
 		};
 
 		struct DetectParams {
 			const float2* x;       // samples; column c starts at 32 c
 			int cols;
+			int batches;           // of 32 columns
 			const float* window;   // 128 Hann coefficients
 			const float2* tw;      // W_128^m, m < 128
 			DetectScratch det;
 		};
 
-		// JammingDetector's STFT and per-column candidates, one warp per column
-		// (grid-stride), the column's transform in registers (Warp128)
-		__global__ void __launch_bounds__(kJamThreads) detect_kernel(DetectParams p) {
-			__shared__ float2 tab[kDetectBins];
+		constexpr int kDetectThreads = 64;
+		constexpr int kMagStride = 137;   // odd: one thread per column reads without conflicts; 9 modulo 32 spreads the four columns of a store
+		constexpr int kDetectWarpBytes = static_cast<int>(sizeof(float2)) * 4 * kOctetTile + static_cast<int>(sizeof(float)) * 32 * (kMagStride + 17);
+
+		// One thread, one column: kMaxCandidates rounds of first-max over the
+		// column's magnitudes (the largest, then the lowest bin holding it, as
+		// std::max_element), each followed by nulling +-3 bins (NullRegion,
+		// jamming_detection.hpp:101-110); then the float mean and unbiased sigma of
+		// the nulled magnitudes with SequentialMeanStdDev's formula (src/math/
+		// mean_stddev.hpp:29-42; the sums in four interleaved parts) and J/N = peak
+		// / sigma.  Candidates with J/N < 6 are erased, the rest kept in order:
+		// kept candidate r of column `col` goes to [r][col] and into the CTA's
+		// round-r occupation histogram.  The maxima of the 16 groups of eight bins
+		// are kept beside the magnitudes, so a round looks at 16 maxima, one group,
+		// and the at most two groups that nulling touched.
+		__device__ __forceinline__ void detect_column(float* mag, float* group, const DetectScratch& d, size_t col, size_t cols,
+			int* s_hist, unsigned int* s_total) {
+			auto group_max = [&](int g) {
+				float m = mag[8 * g];
+#pragma unroll
+				for (int i = 1; i < 8; ++i)
+					m = fmaxf(m, mag[8 * g + i]);
+				group[g] = m;
+			};
+#pragma unroll 4
+			for (int g = 0; g < 16; ++g)
+				group_max(g);
+			int bins[kMaxCandidates];
+			float peaks[kMaxCandidates];
+#pragma unroll
+			for (int r = 0; r < kMaxCandidates; ++r) {
+				float top = group[0];
+				int g = 0;
+#pragma unroll
+				for (int i = 1; i < 16; ++i) {
+					const float m = group[i];
+					g = m > top ? i : g;
+					top = fmaxf(top, m);
+				}
+				int bi = 8 * g + 7;
+#pragma unroll
+				for (int i = 6; i >= 0; --i)
+					bi = mag[8 * g + i] == top ? 8 * g + i : bi;
+				bins[r] = bi;
+				peaks[r] = top;
+#pragma unroll
+				for (int i = -kNullHalfWidth; i <= kNullHalfWidth; ++i)
+					mag[(bi + i) & (kDetectBins - 1)] = 0.0f;
+				if (r + 1 < kMaxCandidates) {
+					const int ga = ((bi - kNullHalfWidth) & (kDetectBins - 1)) >> 3, gb = ((bi + kNullHalfWidth) & (kDetectBins - 1)) >> 3;
+					group_max(ga);
+					if (gb != ga)
+						group_max(gb);
+				}
+			}
+			float q[4] = {0.f, 0.f, 0.f, 0.f}, s[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 8
+			for (int i = 0; i < kDetectBins; i += 4)
+#pragma unroll
+				for (int k = 0; k < 4; ++k) {
+					const float m = mag[i + k];
+					q[k] = __fadd_rn(q[k], __fmul_rn(m, m));
+					s[k] = __fadd_rn(s[k], m);
+				}
+			const float qs = __fadd_rn(__fadd_rn(q[0], q[1]), __fadd_rn(q[2], q[3])), ss = __fadd_rn(__fadd_rn(s[0], s[1]), __fadd_rn(s[2], s[3]));
+			const float fw = static_cast<float>(kDetectBins);
+			const float var = __fdiv_rn(__fsub_rn(qs, __fdiv_rn(__fmul_rn(ss, ss), fw)), static_cast<float>(kDetectBins - 1));
+			const float sigma = __fsqrt_rn(var);
+			int c = 0;
+#pragma unroll
+			for (int r = 0; r < kMaxCandidates; ++r) {
+				// double(peak) / double(sigma) < 6 exactly when peak - 6 sigma < 0
+				// (two floats' double quotient cannot round onto 6 unless it is 6),
+				// and fmaf rounds that difference once, keeping its sign: the
+				// reference's double test without FP64 (a NaN stays, as in
+				// remove_if(jn < threshold)).  The kept J/N is the float quotient.
+				if (!(fmaf(-kJnThreshold, sigma, peaks[r]) < 0.0f)) {
+					d.bins[static_cast<size_t>(c) * cols + col] = static_cast<uint8_t>(bins[r]);
+					d.jn[static_cast<size_t>(c) * cols + col] = __fdiv_rn(peaks[r], sigma);
+					atomicAdd(&s_hist[c * kDetectBins + bins[r]], 1);
+					++c;
+				}
+			}
+			for (int r = c; r < kMaxCandidates; ++r)
+				d.bins[static_cast<size_t>(r) * cols + col] = kNoBin;
+			atomicAdd(s_total, static_cast<unsigned int>(c));
+		}
+
+		// JammingDetector's STFT and per-column candidates: a warp takes batches of
+		// 32 consecutive columns (grid-stride), each octet of lanes eight of them in
+		// a row — a column's samples are the previous one's moved by 32, so only 32
+		// are loaded per column — then each lane one column's candidates.  Bound:
+		// issue, and shared memory for the warps in flight.
+		__global__ void __launch_bounds__(kDetectThreads) detect_kernel(DetectParams p) {
+			extern __shared__ __align__(16) unsigned char raw[];
 			__shared__ int s_hist[kMaxCandidates * kDetectBins];
 			__shared__ unsigned int s_total;
-			for (int e = threadIdx.x; e < kDetectBins; e += blockDim.x)
-				tab[e] = p.tw[e];
 			for (int e = threadIdx.x; e < kMaxCandidates * kDetectBins; e += blockDim.x)
 				s_hist[e] = 0;
 			if (threadIdx.x == 0)
 				s_total = 0;
 			__syncthreads();
-			const int lane = threadIdx.x & 31;
-			Warp128 fft;
-			fft.init(tab, lane);
-			float win[4];
-			int idx[4];
+			const int lane = threadIdx.x & 31, octet = lane >> 3;
+			unsigned char* mine = raw + (threadIdx.x >> 5) * kDetectWarpBytes;
+			float* const mags = reinterpret_cast<float*>(mine + sizeof(float2) * 4 * kOctetTile);
+			float* const groups = mags + 32 * kMagStride;
+			Octet128 fft;
+			fft.init(p.tw, reinterpret_cast<float2*>(mine));
+			float win[16];
 #pragma unroll
-			for (int j = 0; j < 4; ++j) {
-				win[j] = p.window[lane + 32 * j];
-				idx[j] = Warp128::natural(j, lane);
-			}
+			for (int j = 0; j < 16; ++j)
+				win[j] = p.window[fft.l + 8 * j];
 			const int warps = gridDim.x * (blockDim.x >> 5);
-			for (int c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); c < p.cols; c += warps) {
-				const float2* xc = p.x + static_cast<size_t>(c) * 32;
-				float2 v[4];
+			for (int batch = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); batch < p.batches; batch += warps) {
+				const int c0 = batch * 32 + octet * 8;  // the octet's first column
+				// samples of the last column on (clamped: columns past the end repeat it)
+				const float2* x = p.x + static_cast<size_t>(min(c0, p.cols - 1)) * 32 + fft.l;
+				float2 smp[16];
 #pragma unroll
-				for (int j = 0; j < 4; ++j) {
-					const float2 smp = xc[lane + 32 * j];
-					// vec * complex(window, 0) (stft.hpp:55-56): both parts scaled
-					v[j] = c2(__fmul_rn(smp.x, win[j]), __fmul_rn(smp.y, win[j]));
+				for (int j = 0; j < 12; ++j)
+					smp[j + 4] = x[8 * j];
+#pragma unroll 1
+				for (int i = 0; i < 8; ++i) {
+#pragma unroll
+					for (int j = 0; j < 12; ++j)
+						smp[j] = smp[j + 4];
+					if (c0 + i < p.cols) {
+#pragma unroll
+						for (int j = 12; j < 16; ++j)
+							smp[j] = x[32 * i + 8 * j];
+					}
+					float2 v[16];
+#pragma unroll
+					for (int j = 0; j < 16; ++j)  // vec * complex(window, 0) (stft.hpp:55-56): both parts scaled
+						v[j] = c2(__fmul_rn(smp[j].x, win[j]), __fmul_rn(smp[j].y, win[j]));
+					fft.forward(v);
+					float* m = mags + (octet * 8 + i) * kMagStride + fft.l;
+#pragma unroll
+					for (int j = 0; j < 16; ++j)
+						m[8 * j] = __fsqrt_rn(v[j].x * v[j].x + v[j].y * v[j].y);
 				}
-				fft.forward(v, lane);
-				float mv[4];
-#pragma unroll
-				for (int j = 0; j < 4; ++j)
-					mv[j] = magnitude(v[j]);
-				detect_column(mv, idx, p.det, static_cast<size_t>(c), static_cast<size_t>(p.cols), s_hist, &s_total);
+				__syncwarp();
+				const int col = batch * 32 + lane;
+				if (col < p.cols)
+					detect_column(mags + lane * kMagStride, groups + lane * 17, p.det, static_cast<size_t>(col), static_cast<size_t>(p.cols),
+						s_hist, &s_total);
+				__syncwarp();  // the next batch writes the magnitudes
 			}
 			__syncthreads();
 			for (int e = threadIdx.x; e < kMaxCandidates * kDetectBins; e += blockDim.x)
@@ -409,81 +441,113 @@ namespace ugsdr_gpu {
 			const float2* x;       // n input samples
 			uint64_t n;
 			int cols;
-			int slots_per_warp;    // 32-sample output slots per warp
+			int slots_per_octet;   // 32-sample output slots per run
 			const float* window;
 			const float2* tw;      // W_128^m, m < 128
 			float2* out;           // n output samples (not x)
 		};
 
-		// FilterWideband (jse.hpp:70-87) + OverlapAndAdd + resize to n, one warp
-		// per run of 32-sample output slots: it walks the covering columns in
-		// order (its first slot's three predecessors first), re-transforming each
-		// from the samples as the detector did (Warp128), zeroing |.| >= 20,
-		// inverse-transforming and scaling (v / 128) * 2; column i's value j
-		// belongs to slot i + j, so four slot accumulators per lane take the
-		// columns in column order, and slot i is complete after column i.
-		__global__ void __launch_bounds__(kJamThreads) wideband_kernel(WidebandParams p) {
-			__shared__ float2 tab[kDetectBins];
-			for (int e = threadIdx.x; e < kDetectBins; e += blockDim.x)
-				tab[e] = p.tw[e];
-			__syncthreads();
-			const int lane = threadIdx.x & 31;
+		// float(|X|) >= 20 (jse.hpp:43) on the square: the root of the float below
+		// 400 is the first to round to 20
+		constexpr float kWidebandLevel2 = 0x1.8ffffep+8f;
+		constexpr int kWidebandThreads = 128;
+
+		// FilterWideband (jse.hpp:70-87) + OverlapAndAdd + resize to n, eight lanes
+		// per run of 32-sample output slots: they walk the covering columns in
+		// order (the first slot's three predecessors first), re-transforming each
+		// from the samples as the detector did (Octet128; 32 new samples per
+		// column), zeroing |.| >= 20, inverse-transforming and scaling (v / 128) *
+		// 2; a column's samples 32 q .. belong to slot i + q, so four slot
+		// accumulators take the columns in column order, and slot i is complete
+		// after column i.  Bound: issue.
+		__global__ void __launch_bounds__(kWidebandThreads) wideband_kernel(WidebandParams p) {
+			__shared__ __align__(16) float2 tiles[kWidebandThreads / 8 * kOctetTile];
+			const int octet = static_cast<int>(threadIdx.x >> 3);
 			const long long total_slots = static_cast<long long>((p.n + 31) / 32);
-			const long long s0 = (static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5)) * p.slots_per_warp;
-			if (s0 >= total_slots)
-				return;
-			const long long s1 = min(s0 + p.slots_per_warp, total_slots);
-			Warp128 fft;
-			fft.init(tab, lane);
-			float win[4];
+			const long long s0 = (static_cast<long long>(blockIdx.x) * (kWidebandThreads / 8) + octet) * p.slots_per_octet;
+			const long long s1 = min(s0 + p.slots_per_octet, total_slots);
+			Octet128 fft;
+			fft.init(p.tw, tiles + (threadIdx.x >> 5) * (4 * kOctetTile));
+			float win[16];
 #pragma unroll
-			for (int j = 0; j < 4; ++j)
-				win[j] = p.window[lane + 32 * j];
-			const float fw = static_cast<float>(kDetectBins);
-			float2 acc[4];
+			for (int j = 0; j < 16; ++j)
+				win[j] = p.window[fft.l + 8 * j];
+			// slot i + q's sums, samples fft.l + 8 k of the slot
+			float2 acc[4][4];
 #pragma unroll
-			for (int j = 0; j < 4; ++j)
-				acc[j] = c2(0.0f, 0.0f);
-			auto put = [&](long long s, float2 v) {
-				const uint64_t k = static_cast<uint64_t>(s) * 32 + lane;
-				if (k < p.n)
-					p.out[k] = v;
+			for (int q = 0; q < 4; ++q)
+#pragma unroll
+				for (int k = 0; k < 4; ++k)
+					acc[q][k] = c2(0.0f, 0.0f);
+			auto put = [&](long long s, const float2 (&v)[4]) {
+#pragma unroll
+				for (int k = 0; k < 4; ++k) {
+					const uint64_t at = static_cast<uint64_t>(s) * 32 + fft.l + 8 * k;
+					if (at < p.n)
+						p.out[at] = v[k];
+				}
 			};
-			const long long i_lo = max(0LL, s0 - 3);
-			const long long i_hi = min(static_cast<long long>(p.cols) - 1, s1 - 1);
-			for (long long i = i_lo; i <= i_hi; ++i) {
-				const float2* xc = p.x + static_cast<size_t>(i) * 32;
-				float2 v[4];
+			const long long i_lo = s0 - 3;  // columns before the first and past the last add nothing
+			float2 smp[16];
+			{
+				const long long first = max(0LL, min(i_lo, static_cast<long long>(p.cols) - 1));
 #pragma unroll
-				for (int j = 0; j < 4; ++j) {
-					const float2 smp = xc[lane + 32 * j];
-					v[j] = c2(__fmul_rn(smp.x, win[j]), __fmul_rn(smp.y, win[j]));
+				for (int j = 0; j < 12; ++j)
+					smp[j + 4] = p.x[static_cast<size_t>(first) * 32 + fft.l + 8 * j];
+			}
+			// every octet of the warp walks the same number of columns (the
+			// exchanges synchronise the warp)
+			for (int step = 0; step < p.slots_per_octet + 3; ++step) {
+				const long long i = i_lo + step;
+				const bool live = i >= 0 && i < p.cols && i < s1;
+				// the window moves on from the first column that exists
+				if (i > 0) {
+#pragma unroll
+					for (int j = 0; j < 12; ++j)
+						smp[j] = smp[j + 4];
 				}
-				fft.forward(v, lane);
+				else {
 #pragma unroll
-				for (int j = 0; j < 4; ++j)
-					if (magnitude(v[j]) >= kWidebandLevel)
+					for (int j = 0; j < 12; ++j)
+						smp[j] = i == 0 ? smp[j + 4] : smp[j];
+				}
+				if (live) {
+#pragma unroll
+					for (int j = 12; j < 16; ++j)
+						smp[j] = p.x[static_cast<size_t>(i) * 32 + fft.l + 8 * j];
+				}
+				float2 v[16];
+#pragma unroll
+				for (int j = 0; j < 16; ++j)
+					v[j] = c2(__fmul_rn(smp[j].x, win[j]), __fmul_rn(smp[j].y, win[j]));
+				fft.forward(v);
+#pragma unroll
+				for (int j = 0; j < 16; ++j)
+					if (v[j].x * v[j].x + v[j].y * v[j].y >= kWidebandLevel2)
 						v[j] = c2(0.0f, 0.0f);
-				fft.inverse(v, lane);
+				fft.inverse(v);
+				if (live) {
+					// (v / 128) * 2: exact powers of two
 #pragma unroll
-				for (int j = 0; j < 4; ++j) {
-					const long long s = i + j;
-					if (s >= s0 && s < s1) {
-						float2& a = acc[s & 3];
-						a = c2(__fadd_rn(a.x, __fmul_rn(__fdiv_rn(v[j].x, fw), 2.0f)),
-							__fadd_rn(a.y, __fmul_rn(__fdiv_rn(v[j].y, fw), 2.0f)));
-					}
+					for (int q = 0; q < 4; ++q)
+#pragma unroll
+						for (int k = 0; k < 4; ++k) {
+							const float2 y = v[4 * q + k];
+							acc[q][k] = c2(__fadd_rn(acc[q][k].x, __fmul_rn(y.x, 0.015625f)), __fadd_rn(acc[q][k].y, __fmul_rn(y.y, 0.015625f)));
+						}
 				}
-				if (i >= s0) {
-					put(i, acc[i & 3]);
-					acc[i & 3] = c2(0.0f, 0.0f);
+				// slot i is complete; past the last column the synthesis tail (slots
+				// cols .. cols + 2), then the zeros of the resize to n
+				if (i >= s0 && i < s1)
+					put(i, acc[0]);
+#pragma unroll
+				for (int k = 0; k < 4; ++k) {
+					acc[0][k] = acc[1][k];
+					acc[1][k] = acc[2][k];
+					acc[2][k] = acc[3][k];
+					acc[3][k] = c2(0.0f, 0.0f);
 				}
 			}
-			// past the last column: the synthesis tail (slots cols .. cols + 2),
-			// then the zeros of the resize to n
-			const long long len_slots = static_cast<long long>(p.cols) + 3;
-			for (long long s = max(s0, static_cast<long long>(p.cols)); s < s1; ++s)
-				put(s, s < len_slots ? acc[s & 3] : c2(0.0f, 0.0f));
 		}
 
 		struct NullRange {
@@ -607,28 +671,26 @@ namespace ugsdr_gpu {
 			note_launch(ctx, 2);
 		}
 
-		int grid_for_warps(ugsdr_ctx* ctx, long long warps) {
-			const long long per_cta = kJamThreads / 32;
-			return static_cast<int>(std::max<long long>(1, std::min<long long>((warps + per_cta - 1) / per_cta,
-				static_cast<long long>(ctx->sm_count) * 64)));
-		}
-
 		// FilterWideband + OverlapAndAdd + resize to n, fused: x -> out
 		void wideband_device(ugsdr_ctx* ctx, const float2* x, size_t n, float2* out) {
-			constexpr int kSlotsPerWarp = 64;
 			WidebandParams p{};
 			p.x = x;
 			p.n = n;
 			p.cols = static_cast<int>(stft_columns(n, kDetectWindow, kDetectOverlap));
-			p.slots_per_warp = kSlotsPerWarp;
+			// runs of up to 64 slots (each walks three more columns), of the length
+			// that makes whole waves of the CTAs three of which share an SM
+			const long long slots = static_cast<long long>((n + 31) / 32);
+			const long long wave = static_cast<long long>(ctx->sm_count) * 3 * (kWidebandThreads / 8);  // octets
+			const long long waves = (slots + 64 * wave - 1) / (64 * wave);
+			p.slots_per_octet = static_cast<int>(std::max<long long>(8, (slots + waves * wave - 1) / (waves * wave)));
 			p.window = hann_window(ctx, kDetectWindow);
 			p.tw = get_plan(ctx, kDetectWindow).tw;
 			p.out = out;
-			const long long warps = (static_cast<long long>((n + 31) / 32) + kSlotsPerWarp - 1) / kSlotsPerWarp;
-			const long long ctas = (warps + kJamThreads / 32 - 1) / (kJamThreads / 32);
+			const long long octets = (slots + p.slots_per_octet - 1) / p.slots_per_octet;
+			const long long ctas = (octets + kWidebandThreads / 8 - 1) / (kWidebandThreads / 8);
 			require(ctas < (1LL << 31), "signal too long");
 			KernelTimer timer(ctx, "jam_wideband");
-			wideband_kernel<<<static_cast<unsigned>(ctas), kJamThreads, 0, ctx->stream>>>(p);
+			wideband_kernel<<<static_cast<unsigned>(ctas), kWidebandThreads, 0, ctx->stream>>>(p);
 			note_launch(ctx);
 		}
 
@@ -657,49 +719,59 @@ namespace ugsdr_gpu {
 		// by frequency = bin * fs / w, which orders as the bins do, so the
 		// reference's walk over the map is a walk over occupied bins in
 		// increasing order of the round's histogram.
-		__global__ void decide_kernel(DetectScratch d, unsigned long long cols) {
-			if (threadIdx.x != 0)
-				return;
+		// One warp per round, lane l on bins l, l + 32, ...; the walk's state at a
+		// bin follows from the ballots of the bins below it.
+		__global__ void __launch_bounds__(32 * kMaxCandidates) decide_kernel(DetectScratch d, unsigned long long cols) {
 			const int rounds = static_cast<int>(*d.total / cols);
-			for (int i = 0; i < rounds; ++i) {
-				const int* occ = d.hist + i * kDetectBins;
-				double quantity = 0;
-				int occupied = 0;
-				for (int b = 0; b < kDetectBins; ++b)
-					if (occ[b]) {
-						quantity += occ[b];
-						++occupied;
-					}
-				int narrow = -1, wide = -1, first = -1;
-				unsigned long long cnt_wideband = 0;
-				for (int b = 0; b < kDetectBins; ++b) {
-					if (!occ[b])
-						continue;
-					if (first < 0)
-						first = b;
-					const double probability = occ[b] / quantity;
-					if (probability >= kProbability) {
-						narrow = b;
-						break;
-					}
-					if (probability >= kProbability / static_cast<double>(occupied)) {
-						++cnt_wideband;
-						wide = b;
-					}
+			if (threadIdx.x == 0)
+				*d.rounds = rounds;
+			const int i = threadIdx.x >> 5, lane = threadIdx.x & 31;
+			if (i >= rounds)
+				return;
+			constexpr int J = kDetectBins / 32;
+			int occ[J], sum = 0, occupied = 0;
+			unsigned occupied_mask[J];
+#pragma unroll
+			for (int j = 0; j < J; ++j) {
+				occ[j] = d.hist[i * kDetectBins + j * 32 + lane];
+				sum += occ[j];
+				occupied_mask[j] = __ballot_sync(0xffffffffu, occ[j] != 0);
+				occupied += __popc(occupied_mask[j]);
+			}
+			const double quantity = static_cast<double>(__reduce_add_sync(0xffffffffu, sum));
+			int narrow = -1, wide = -1, first = -1;
+			unsigned long long cnt_wideband = 0;
+#pragma unroll
+			for (int j = 0; j < J; ++j) {
+				const double probability = occ[j] / quantity;
+				const unsigned sure = __ballot_sync(0xffffffffu, occ[j] != 0 && probability >= kProbability);
+				unsigned many = __ballot_sync(0xffffffffu, occ[j] != 0 && probability >= kProbability / static_cast<double>(occupied));
+				if (first < 0 && occupied_mask[j])
+					first = j * 32 + __ffs(static_cast<int>(occupied_mask[j])) - 1;
+				if (narrow >= 0)
+					continue;  // the walk ended below these bins
+				if (sure) {
+					narrow = j * 32 + __ffs(static_cast<int>(sure)) - 1;
+					many &= (1u << (narrow & 31)) - 1u;
 				}
-				if (wide < 0)
-					wide = first;  // the reference's pointer starts at the map's first entry
+				if (many) {
+					cnt_wideband += __popc(many);
+					wide = j * 32 + 31 - __clz(static_cast<int>(many));
+				}
+			}
+			if (wide < 0)
+				wide = first;  // the reference's pointer starts at the map's first entry
+			if (lane == 0) {
 				d.picks[2 * i] = narrow;
 				// one occupied bin makes the bound 0: reported as wideband too
 				d.picks[2 * i + 1] = cnt_wideband >= static_cast<unsigned long long>(occupied * kProbability) ? wide : -1;
 				d.quantity[i] = quantity;
 			}
-			*d.rounds = rounds;
 		}
 
 		// The reported J/N of each pick: the mean of the round's candidate J/N
 		// at that bin.  Per-CTA partial sums over a fixed column split, combined
-		// in CTA order by the last CTA, which also writes the detection list —
+		// in a fixed tree by the last CTA, which also writes the detection list —
 		// deterministic, within rounding of the reference's column-order sum.
 		__global__ void __launch_bounds__(kJamThreads) jn_sum_kernel(DetectScratch d, unsigned long long cols, double fs) {
 			__shared__ double scratch[32];
@@ -727,7 +799,7 @@ namespace ugsdr_gpu {
 				s_last = atomicAdd(d.done, 1u) == gridDim.x - 1;
 			}
 			__syncthreads();
-			if (!s_last || threadIdx.x != 0)
+			if (!s_last)
 				return;
 			__threadfence();
 			int n = 0;
@@ -736,16 +808,22 @@ namespace ugsdr_gpu {
 					const int b = d.picks[2 * i + k];
 					if (b < 0 || n >= kMaxDetections)
 						continue;
-					double sum = 0;
-					for (unsigned int g = 0; g < gridDim.x; ++g)
-						sum += __ldcg(d.partials + g * kMaxDetections + 2 * i + k);
+					double part = 0;
+					for (unsigned int g = threadIdx.x; g < gridDim.x; g += blockDim.x)
+						part += __ldcg(d.partials + g * kMaxDetections + 2 * i + k);
+					const double sum = block_sum(part, scratch);
+					if (threadIdx.x != 0) {
+						++n;
+						continue;
+					}
 					Detection& out = d.list->d[n++];
 					out.type = k == 0 ? UGSDR_INTERFERENCE_NARROWBAND : UGSDR_INTERFERENCE_WIDEBAND;
 					out.bin = b;
 					out.frequency = static_cast<double>(b) * fs / static_cast<double>(kDetectBins);
 					out.jn = sum / d.quantity[i];
 				}
-			d.list->n = n;
+			if (threadIdx.x == 0)
+				d.list->n = n;
 		}
 
 		// detector over device samples x (n): STFT + candidates, decisions and
@@ -760,15 +838,20 @@ namespace ugsdr_gpu {
 			DetectParams dp{};
 			dp.x = x;
 			dp.cols = static_cast<int>(cols);
+			dp.batches = static_cast<int>((cols + 31) / 32);
 			dp.window = hann_window(ctx, kDetectWindow);
 			dp.tw = get_plan(ctx, kDetectWindow).tw;
 			dp.det = d;
 			{
 				KernelTimer timer(ctx, "jam_stft_detect");
-				detect_kernel<<<grid_for_warps(ctx, static_cast<long long>(cols)), kJamThreads, 0, ctx->stream>>>(dp);
+				constexpr int kWarps = kDetectThreads / 32;
+				const size_t smem = static_cast<size_t>(kWarps) * kDetectWarpBytes;
+				UG_CUDA(cudaFuncSetAttribute(detect_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+				const int ctas = std::min((dp.batches + kWarps - 1) / kWarps, ctx->sm_count * 16);
+				detect_kernel<<<ctas, kDetectThreads, smem, ctx->stream>>>(dp);
 			}
 			note_launch(ctx);
-			decide_kernel<<<1, 32, 0, ctx->stream>>>(d, cols);
+			decide_kernel<<<1, 32 * kMaxCandidates, 0, ctx->stream>>>(d, cols);
 			jn_sum_kernel<<<kSumCtas, kJamThreads, 0, ctx->stream>>>(d, cols, fs);
 			note_launch(ctx, 2);
 			DetectionList host{};
