@@ -15,6 +15,7 @@
 #include <cmath>
 #include <cstring>
 #include <functional>
+#include <limits>
 #include <numeric>
 #include <tuple>
 #include <vector>
@@ -996,10 +997,64 @@ namespace ugsdr_gpu {
 	}
 
 	namespace {
-		// The single-CTA kernels' plan of block size n: radices, the pass twiddle
-		// tables (per pass s >= 1 W_N^{r k N / (NS R)} at [r - 1][k]), threads and
-		// CTAs per row.  n_pass = 0: a size those kernels don't take (a lone
-		// pass, or tiles beyond shared memory).
+		// The pass twiddle tables of the single-CTA kernels' radices: per pass
+		// s >= 1 W_N^{r k N / (NS R)} at [r - 1][k].  One plan per size, one table.
+		const float2* pass_tables(ugsdr_ctx* ctx, const SmallPlan& p) {
+			auto& slot = ctx->pass_tables[p.n];
+			if (!slot) {
+				std::vector<float2> t;
+				const double two_pi = 2.0 * 3.14159265358979323846;
+				int ns = p.radix[0];
+				for (int s = 1; s < p.n_pass; ++s) {
+					const int step = p.n / (ns * p.radix[s]);
+					for (int r = 1; r < p.radix[s]; ++r)
+						for (int k = 0; k < ns; ++k) {
+							const double a = two_pi * static_cast<double>(static_cast<int64_t>(r) * k * step % p.n) / p.n;
+							t.push_back(c2(static_cast<float>(std::cos(a)), static_cast<float>(-std::sin(a))));
+						}
+					ns *= p.radix[s];
+				}
+				auto buf = std::make_unique<DevBuf>();
+				buf->reserve(sizeof(float2) * t.size());
+				UG_CUDA(cudaMemcpy(buf->ptr, t.data(), sizeof(float2) * t.size(), cudaMemcpyHostToDevice));
+				UG_CUDA(cudaStreamSynchronize(nullptr));  // in place before any stream reads it
+				slot = std::move(buf);
+			}
+			return slot->as<float2>();
+		}
+
+		// CTAs per row (a cluster of eight at most): the cheapest of rows x split
+		// CTAs, each with its share of the K blocks and two blocks' worth of
+		// setup and summing.  An SM holds `cap` CTAs and runs 512 / threads of
+		// them at the pace of one; beyond `cap`, the mean of whole rounds and of
+		// a steady flow with three quarters of a CTA for its tail; the most
+		// CTAs among equals.  Fitted to 8
+		// sizes of 1,023 to 5,000 points, 21 to 2,592 rows, K 2 to 20: the
+		// rule's pick is within 10 % of the best split at most shapes (168 rows x
+		// 4 of 5,000 points: 36 us unsplit, 49 by two; 84 x 10: 57, 45, 38 by three).
+		int wave_split(ugsdr_ctx* ctx, int rows, int k_blocks, int threads, int cap) {
+			const double free = 512.0 / threads;
+			auto round = [&](int ctas) { return ctas ? std::max(1.0, ctas / free) : 0.0; };
+			int best = 1;
+			double best_cost = 1e300;
+			for (int s = 1; s <= std::min(8, k_blocks); ++s) {
+				const int share = (k_blocks + s - 1) / s;
+				const double mean = static_cast<double>(rows) * s / ctx->sm_count;
+				const int most = static_cast<int>(std::ceil(mean));
+				double load = most / cap * round(cap) + round(most % cap);
+				if (most > cap)
+					load = 0.5 * (load + (mean + 0.75) / free);
+				if (load * (share + 2) <= best_cost) {
+					best_cost = load * (share + 2);
+					best = s;
+				}
+			}
+			return best;
+		}
+
+		// The single-CTA kernels' plan of block size n: radices, twiddle tables,
+		// threads and CTAs per row.  n_pass = 0: a size those kernels don't take
+		// (a lone pass, or tiles beyond shared memory).
 		SmallPlan small_plan(ugsdr_ctx* ctx, int n, int rows, int k_blocks, bool one_sided) {
 			const FftPlanDesc& d = get_plan(ctx, n);
 			SmallPlan p{};
@@ -1011,27 +1066,7 @@ namespace ugsdr_gpu {
 				p.n_pass = 0;
 				return p;
 			}
-			auto& slot = ctx->pass_tables[n];
-			if (!slot) {
-				std::vector<float2> t;
-				const double two_pi = 2.0 * 3.14159265358979323846;
-				int ns = d.radix[0];
-				for (int s = 1; s < d.n_pass; ++s) {
-					const int step = n / (ns * d.radix[s]);
-					for (int r = 1; r < d.radix[s]; ++r)
-						for (int k = 0; k < ns; ++k) {
-							const double a = two_pi * static_cast<double>(static_cast<int64_t>(r) * k * step % n) / n;
-							t.push_back(c2(static_cast<float>(std::cos(a)), static_cast<float>(-std::sin(a))));
-						}
-					ns *= d.radix[s];
-				}
-				auto buf = std::make_unique<DevBuf>();
-				buf->reserve(sizeof(float2) * t.size());
-				UG_CUDA(cudaMemcpy(buf->ptr, t.data(), sizeof(float2) * t.size(), cudaMemcpyHostToDevice));
-				UG_CUDA(cudaStreamSynchronize(nullptr));  // in place before any stream reads it
-				slot = std::move(buf);
-			}
-			p.tables = slot->as<float2>();
+			p.tables = pass_tables(ctx, p);
 			// threads: the most (up to 256) whose idle lanes in the passes' last
 			// rounds cost no more than a tenth over the best choice
 			auto cost = [&](int t) {
@@ -1047,13 +1082,9 @@ namespace ugsdr_gpu {
 			for (int t = 64; t <= kSmallThreads; t += 32)
 				if (cost(t) <= 1.1 * best)
 					p.threads = t;
-			// rows that leave CTA slots empty: the K blocks of a row go to several
-			// CTAs (a cluster of eight at most), the same number of blocks each
-			const int regs = !one_sided ? 255 : *std::max_element(p.radix, p.radix + p.n_pass) <= 25 ? 80 : 128;
-			const int per_sm = std::max(1, std::min(kSmallSmem / (small_inv_bytes(p) + 1024), 65536 / (regs * p.threads)));
-			int split = std::min({8, k_blocks, std::max(1, ctx->sm_count * per_sm / std::max(rows, 1))});
-			split = (k_blocks + (k_blocks + split - 1) / split - 1) / ((k_blocks + split - 1) / split);
-			p.split = split;
+			// resident CTAs: shared memory, and 128 registers a thread
+			const int cap = std::min(kSmallSmem / (small_inv_bytes(p) + 1024), 512 / p.threads);
+			p.split = wave_split(ctx, rows, k_blocks, p.threads, std::max(1, cap));
 			return p;
 		}
 
@@ -1093,18 +1124,18 @@ namespace ugsdr_gpu {
 				}
 			}
 			note_launch(ctx);
-			// a, b, the N-float accumulator, the pass tables (N entries)
-			const size_t smem_i = 2 * sizeof(float2) * F::N + sizeof(float) * F::N + sizeof(float2) * F::N + 16;
 			KernelTimer timer(ctx, "acq_inverse");
-			auto inverse = [&](auto kernel) {
-				set_smem(kernel, smem_i);
-				kernel<<<nd * n_codes, kThreads, smem_i, ctx->stream>>>(p);
-			};
+			SmallPlan plan{};
+			plan.n = F::N;
+			plan.n_pass = 3;
+			plan.radix[0] = 25;
+			plan.radix[1] = 10;
+			plan.radix[2] = 16;
+			plan.tables = pass_tables(ctx, plan);
+			plan.threads = kSmallThreads;
+			plan.split = wave_split(ctx, nd * n_codes, k, kSmallThreads, 3);
 			// one-sided spectra: pass 0 reads only the lower half of Z
-			if (p.one_sided && !std::getenv("UGSDR_NO_PRUNE"))
-				inverse(acq_inverse_static_kernel<F, true>);
-			else
-				inverse(acq_inverse_static_kernel<F>);
+			launch_inv_4000(p, plan, p.one_sided && !std::getenv("UGSDR_NO_PRUNE"), nd * n_codes, ctx->stream);
 			note_launch(ctx);
 		}
 	}

@@ -203,57 +203,6 @@ namespace ugsdr_gpu {
 		F::template run_hooked<false, true>(a, b, plan, 1, F::N, load, emit);
 	}
 
-	struct SmallInvLoad {
-		const float2* x;
-		const float2* code;
-		int half, one_sided;
-		__device__ __forceinline__ float2 operator()(int, int i) const {
-			return (one_sided && i > half) ? c2(0.f, 0.f) : cmul(__ldg(x + i), __ldg(code + i));
-		}
-	};
-	struct SmallInvEmit {
-		float* acc;
-		float inv_n, post;
-		int stat;
-		template <int R, int NS>
-		__device__ __forceinline__ void put(int, int base, const float2 (&v)[R]) const {
-#pragma unroll
-			for (int r = 0; r < R; ++r)
-				acc[base + r * NS] += stat_of(cscale(cscale(v[r], inv_n), post), stat);
-		}
-	};
-	// one-sided: Z is zero above N/2, so pass 0 reads only its live inputs
-	template <int ZF>
-	struct SmallInvLoadZ : SmallInvLoad {
-		static constexpr int kZeroFrom = ZF;
-	};
-	// grid: codes x Doppler bins; unfolded rows (m == N) only.  Each thread
-	// owns the same last-pass outputs in every block, so its accumulator
-	// entries need no barrier between blocks.  HALF: one-sided spectra (the
-	// pruned pass 0 of SmallInvLoadZ)
-	template <class F, bool HALF = false>
-	__global__ void __launch_bounds__(256) acq_inverse_static_kernel(AcqParams p) {
-		extern __shared__ float2 smem[];
-		float2* a = smem;
-		float2* b = smem + F::N;
-		float* acc = reinterpret_cast<float*>(smem + 2 * F::N);
-		const FftPlanDev plan = F::prepare(p.plan, acc + F::N);
-		const int row = blockIdx.x;
-		const int c = row % p.n_codes;
-		const int d = row / p.n_codes;
-		for (int i = threadIdx.x; i < F::N; i += blockDim.x)
-			acc[i] = 0.f;
-		__syncthreads();
-		const SmallInvEmit emit{acc, 1.0f / static_cast<float>(F::N), p.one_sided ? 2.0f : 1.0f, p.stat};
-		for (int blk = 0; blk < p.k_blocks; ++blk) {
-			const SmallInvLoadZ<HALF ? F::N / 2 + 1 : F::N> load{SmallInvLoad{p.spectra + (static_cast<size_t>(d) * p.k_blocks + blk) * F::N,
-				p.codes[c], F::N / 2, p.one_sided}};
-			F::template run_hooked<true, true>(a, b, plan, 1, F::N, load, emit);
-			__syncthreads();  // pass 0 of the next block rewrites the tiles
-		}
-		reduce_cell(acc, F::N, p.cells + static_cast<size_t>(c) * p.n_doppler + p.d_base + d);
-	}
-
 	// ------------------------------------------------------------- forward
 	template <int ST>
 	__device__ __forceinline__ float2 fwd_load(const BatchedParams& p, int item, int64_t i, const float* lut) {

@@ -112,11 +112,15 @@ namespace ugsdr_gpu {
 				for (int r = 1; r < P::R1; ++r)
 					v[r] = cmulc(v[r], tw1[(r - 1) * P::R0 + j1]);
 				Dft<P::R1, true>::run(v);
+				float m[P::R1];
 #pragma unroll
-				for (int r = 0; r < P::R1; ++r) {
-					const float m2 = v[r].x * v[r].x + v[r].y * v[r].y;
-					acc[r] += STAT ? m2 : sqrt_approx(m2);
-				}
+				for (int r = 0; r < P::R1; ++r)
+					m[r] = v[r].x * v[r].x + v[r].y * v[r].y;
+				if constexpr (!STAT)
+					roots(m);
+#pragma unroll
+				for (int r = 0; r < P::R1; ++r)
+					acc[r] += m[r];
 			}
 		}
 		// scale once: |s y| = s |y| with s = 2 / N one-sided (1 / N two-sided)

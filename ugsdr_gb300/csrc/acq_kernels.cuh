@@ -197,9 +197,42 @@ namespace ugsdr_gpu {
 		asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
 		return r;
 	}
+	// |v| of a butterfly's R outputs from their squares.  The instruction above
+	// is four where its input may be subnormal (compare, scale, root, scale
+	// back), so the smallest square decides once for all R of them: from the
+	// smallest normal number on, the flushing form is one instruction and
+	// returns the same bits.  NaN takes either path to NaN.
+	template <int R>
+	__device__ __forceinline__ void roots(float (&m)[R]) {
+		float lo = m[0];
+#pragma unroll
+		for (int r = 1; r < R; ++r)
+			lo = fminf(lo, m[r]);
+		if (lo >= 1.17549435e-38f) {
+#pragma unroll
+			for (int r = 0; r < R; ++r)
+				asm("sqrt.approx.ftz.f32 %0, %0;" : "+f"(m[r]));
+		}
+		else {
+#pragma unroll
+			for (int r = 0; r < R; ++r)
+				m[r] = sqrt_approx(m[r]);
+		}
+	}
 	__device__ __forceinline__ float stat_of(float2 v, int stat) {
 		const float q = v.x * v.x + v.y * v.y;
 		return stat ? q : sqrt_approx(q);
+	}
+	// the statistic of a butterfly's outputs, scaled
+	template <int R>
+	__device__ __forceinline__ void stats_of(const float2 (&v)[R], float scale, int stat, float (&m)[R]) {
+#pragma unroll
+		for (int r = 0; r < R; ++r) {
+			const float2 y = cscale(v[r], scale);
+			m[r] = y.x * y.x + y.y * y.y;
+		}
+		if (!stat)
+			roots(m);
 	}
 
 	// block-wide first-max / sum reduction helpers

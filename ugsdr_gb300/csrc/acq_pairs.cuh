@@ -253,11 +253,15 @@ namespace ugsdr_gpu {
 						v[r] = cmulc(v[r], wk[r]);
 					Dft<R, true>::run(v);
 					float* ac = acc + u * lay.accs;
+					float m[R];
 #pragma unroll
-					for (int r = 0; r < R; ++r) {
-						const float m2 = v[r].x * v[r].x + v[r].y * v[r].y;
-						ac[r] += STAT ? m2 : sqrt_approx(m2);
-					}
+					for (int r = 0; r < R; ++r)
+						m[r] = v[r].x * v[r].x + v[r].y * v[r].y;
+					if constexpr (!STAT)
+						roots(m);
+#pragma unroll
+					for (int r = 0; r < R; ++r)
+						ac[r] += m[r];
 				}
 			});
 			__syncthreads();  // the next block's pass 0 rewrites the tile

@@ -29,6 +29,19 @@ namespace ugsdr_gpu {
 		int split;             // CTAs per row (inverse)
 	};
 
+	// Three passes in place (the inverse): pass 0's butterfly j leaves output
+	// k0 at j s0 + (j / R2) pad + k0; the middle pass takes j = j1 + R2 r, r <
+	// R1, of one (j1, k0) and leaves k1 at (j1 + R2 k1, k0), so no thread waits
+	// between its reads and its writes; the last pass takes the R2 values j1 of
+	// one (k0, k1), whose output k2 is element k0 + R0 k1 + R0 R1 k2.  s0 is
+	// odd (pass 0's stores) and a group of R2 rows padded so that the last
+	// pass's lanes run on through the banks from one k1 to the next.
+	struct InPlace {
+		int s0, pad, group, elems;
+		UG_HD constexpr InPlace(int r0, int r1, int r2)
+			: s0(r0 | 1), pad(((r0 - s0 * r2) % 16 + 16) % 16), group(s0 * r2 + pad), elems(group * r1) {}
+	};
+
 	// elements of pass 0's tile
 	UG_HD int small_tile(const SmallPlan& plan) { return plan.n + (plan.radix[0] % 2 == 0 ? plan.n / plan.radix[0] : 0); }
 	// the tiles of a transform (a second one with a middle pass), bytes
@@ -36,7 +49,8 @@ namespace ugsdr_gpu {
 		return static_cast<int>(sizeof(float2)) * (small_tile(plan) + (plan.n_pass > 2 ? plan.n : 0));
 	}
 	inline int small_inv_bytes(const SmallPlan& plan) {
-		return static_cast<int>(sizeof(float2)) * ((plan.n + 1) / 2) + small_tiles_bytes(plan);
+		return static_cast<int>(sizeof(float2)) * ((plan.n + 1) / 2) + (plan.n_pass == 3
+			? static_cast<int>(sizeof(float2)) * InPlace(plan.radix[0], plan.radix[1], plan.radix[2]).elems : small_tiles_bytes(plan));
 	}
 	// every kernel's limit, set to it always: a context with smaller blocks
 	// never lowers it under another's launch
@@ -48,6 +62,8 @@ namespace ugsdr_gpu {
 	void launch_fwd_small_wide(const AcqParams& p, const SmallPlan& plan, int sample_type, int items, cudaStream_t stream);
 	void launch_inv_small25(const AcqParams& p, const SmallPlan& plan, int rows, cudaStream_t stream);
 	void launch_inv_small32(const AcqParams& p, const SmallPlan& plan, int rows, cudaStream_t stream);
+	// blocks of 4,000 points as 25 x 10 x 16
+	void launch_inv_4000(const AcqParams& p, const SmallPlan& plan, bool half, int rows, cudaStream_t stream);
 
 	// Runs the passes after the first: `a` holds pass 0's output (padded by one
 	// element per butterfly when its radix is even), middle passes ping-pong
@@ -163,11 +179,45 @@ namespace ugsdr_gpu {
 		});
 	}
 
+	// Distributed shared memory: adds the n accumulators of a cluster's `split`
+	// CTAs into the first one's, in order; true in that CTA.  Every CTA sums its
+	// share of the n (a CTA alone reading the others' waits a round trip per
+	// element and CTA: half the kernel's time at 168 rows of 2,500 points).
+	__device__ __forceinline__ bool cluster_sum(float* acc, int n, int split, int part) {
+		asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+		const uint32_t mine = static_cast<uint32_t>(__cvta_generic_to_shared(acc));
+		uint32_t at[8];
+#pragma unroll
+		for (int o = 0; o < 8; ++o)
+			if (o < split)
+				asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at[o]) : "r"(mine), "r"(o));
+		for (int i = part * blockDim.x + threadIdx.x; i < n; i += split * blockDim.x) {
+			float v[8];
+#pragma unroll
+			for (int o = 0; o < 8; ++o)
+				if (o < split)
+					asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v[o]) : "r"(at[o] + 4u * i) : "memory");
+			float s = v[0];
+#pragma unroll
+			for (int o = 1; o < 8; ++o)
+				if (o < split)
+					s += v[o];
+			asm volatile("st.shared::cluster.f32 [%0], %1;" :: "r"(at[0] + 4u * i), "f"(s) : "memory");
+		}
+		asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+		return part == 0;
+	}
+
 	// grid: (rows x split) CTAs in clusters of `split`; unfolded rows (m == N).
+	// Three passes run in place (InPlace) in one tile; the two tiles they took
+	// before left two CTAs per SM from 4,000 points on: 672 rows x 10 blocks of
+	// 4,092 points 307 -> 188 us, of 5,000 380 -> 178.  Two CTAs' worth of
+	// registers (128 a thread): at 80 radices from 12 on spill, 672 x 10 of
+	// 3,000 points 139 us against 110.
 	// HALF: one-sided spectra (Z is zero above N / 2: pass 0 reads R / 2 + 1 of
 	// its R inputs)
 	template <int MAXR, bool HALF>
-	__global__ void __launch_bounds__(kSmallThreads, !HALF ? 1 : MAXR <= 25 ? 3 : 2) acq_inv_small_kernel(const __grid_constant__ AcqParams p,
+	__global__ void __launch_bounds__(kSmallThreads, HALF ? 2 : 1) acq_inv_small_kernel(const __grid_constant__ AcqParams p,
 		const __grid_constant__ SmallPlan plan) {
 		extern __shared__ float2 smem[];
 		const int n = plan.n;
@@ -186,12 +236,15 @@ namespace ugsdr_gpu {
 		// the last pass reads the tile that the next block's first pass rewrites
 		// unless a middle pass (and its barrier) lies between
 		const bool fence = (plan.n_pass & 1) == 0;
+		const bool three = plan.n_pass == 3;
+		const int r0 = plan.radix[0], r1 = plan.radix[1], r2 = three ? plan.radix[2] : 1;
+		const InPlace ip(r0, r1, r2);
+		const float inv_r0 = 1.0f / static_cast<float>(r0), inv_r2 = 1.0f / static_cast<float>(r2);
 		for (int blk = part; blk < p.k_blocks; blk += plan.split) {
 			const float2* x = p.spectra + (static_cast<size_t>(d) * p.k_blocks + blk) * n;
 			with_radix<MAXR>(plan.radix[0], [&](auto rc) {
 				constexpr int R = decltype(rc)::value;
 				constexpr int RL = HALF ? R / 2 + 1 : R;
-				constexpr int PAD = (R & 1) ^ 1;
 				const int nb = n / R;
 				for (int u = threadIdx.x; u < nb; u += blockDim.x) {
 					float2 v[R];
@@ -207,44 +260,166 @@ namespace ugsdr_gpu {
 						DftPruned<R, true, RL>::run(v);
 					else
 						Dft<R, true>::run(v);
-					float2* o = a + u * (R + PAD);
+					float2* o = a + u * (R | 1) + (three ? fdiv(u, inv_r2) * ip.pad : 0);
 #pragma unroll
 					for (int r = 0; r < R; ++r)
 						o[r] = v[r];
 				}
 			});
 			__syncthreads();
+			if (three) {
+				with_radix<MAXR>(r1, [&](auto rc) {
+					constexpr int R = decltype(rc)::value;
+					for (int u = threadIdx.x; u < r0 * r2; u += blockDim.x) {  // u = k0 + R0 j1
+						const int j1 = fdiv(u, inv_r0), k0 = u - j1 * r0;
+						float2* e = a + j1 * ip.s0 + k0;
+						const float2* w = plan.tables + k0;
+						float2 v[R];
+#pragma unroll
+						for (int r = 0; r < R; ++r)
+							v[r] = e[r * ip.group];
+#pragma unroll
+						for (int r = 1; r < R; ++r)
+							v[r] = cmulc(v[r], __ldg(w + (r - 1) * r0));
+						Dft<R, true>::run(v);
+#pragma unroll
+						for (int r = 0; r < R; ++r)
+							e[r * ip.group] = v[r];
+					}
+				});
+				__syncthreads();
+				with_radix<MAXR>(r2, [&](auto rc) {
+					constexpr int R = decltype(rc)::value;
+					const int ns = r0 * r1;
+					for (int u = threadIdx.x; u < ns; u += blockDim.x) {  // u = k0 + R0 k1
+						const int k1 = fdiv(u, inv_r0);
+						const float2* e = a + k1 * ip.group + (u - k1 * r0);
+						const float2* w = plan.tables + r0 * (r1 - 1) + u;
+						float2 v[R];
+#pragma unroll
+						for (int r = 0; r < R; ++r)
+							v[r] = e[r * ip.s0];
+#pragma unroll
+						for (int r = 1; r < R; ++r)
+							v[r] = cmulc(v[r], __ldg(w + (r - 1) * ns));
+						Dft<R, true>::run(v);
+						float m[R];
+						stats_of(v, scale, stat, m);
+#pragma unroll
+						for (int r = 0; r < R; ++r)
+							acc[u + r * ns] += m[r];
+					}
+				});
+				__syncthreads();  // the next block's pass 0 rewrites the tile
+				continue;
+			}
 			small_passes<MAXR, true>(a, b, plan, [&](int u, int ns, auto& v, auto rc) {
 				constexpr int R = decltype(rc)::value;
+				float m[R];
+				stats_of(v, scale, stat, m);
 #pragma unroll
 				for (int r = 0; r < R; ++r)
-					acc[u + r * ns] += stat_of(cscale(v[r], scale), stat);
+					acc[u + r * ns] += m[r];
 			});
 			if (fence)
 				__syncthreads();
 		}
-		if (plan.split > 1) {
-			// distributed shared memory: the first CTA of the cluster adds the others'
-			// accumulators in order (every CTA arrives once before and once after)
-			asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-			if (part == 0) {
-				const uint32_t mine = static_cast<uint32_t>(__cvta_generic_to_shared(acc));
-				for (int o = 1; o < plan.split; ++o) {
-					uint32_t theirs;
-					asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(theirs) : "r"(mine), "r"(o));
-					for (int i = threadIdx.x; i < n; i += blockDim.x) {
-						float v;
-						asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(theirs + 4u * i) : "memory");
-						acc[i] += v;
-					}
-				}
-			}
-			asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-			if (part != 0)
-				return;
-		}
+		if (plan.split > 1 && !cluster_sum(acc, n, plan.split, part))
+			return;
 		__syncthreads();
 		reduce_cell(acc, n, p.cells + static_cast<size_t>(c) * p.n_doppler + p.d_base + d);
+	}
+
+	// The same for N = R0 R1 R2 with every pass compiled in.  At 4,000 points
+	// 48 KB a CTA, so registers decide (three CTAs per SM); two tiles and a
+	// staged twiddle table (112 KB) left two: 672 rows x 10 blocks 128 -> 90 us.
+	// Bound: the L1 / shared-memory data pipe (60 %), issue (51 %) and the
+	// barriers between the passes.
+	template <int R0, int R1, int R2, bool HALF>
+	__global__ void __launch_bounds__(kSmallThreads, 3) acq_inv_three_kernel(const __grid_constant__ AcqParams p,
+		const __grid_constant__ SmallPlan plan) {
+		constexpr int N = R0 * R1 * R2, NB0 = N / R0, NB1 = N / R1, NB2 = N / R2;
+		static_assert(R0 % 2 == 1, "rows of R0 elements: the middle pass's u runs along them");
+		static_assert(NB0 <= kSmallThreads && NB1 <= 2 * kSmallThreads && NB2 <= kSmallThreads, "butterflies per thread");
+		constexpr int RL = HALF ? R0 / 2 + 1 : R0;
+		constexpr InPlace ip(R0, R1, R2);
+		constexpr int GS = ip.group;
+		extern __shared__ float2 smem[];
+		float2* const t = smem;
+		float* const acc = reinterpret_cast<float*>(smem + ip.elems);
+		const int tid = threadIdx.x;
+		float2* const first = t + tid * R0 + tid / R2 * ip.pad;
+		const float2* const last = t + tid / R0 * GS + tid % R0;
+		const int row = blockIdx.x / plan.split;
+		const int part = blockIdx.x - row * plan.split;
+		const int c = row % p.n_codes;
+		const int d = row / p.n_codes;
+		const float2* code = p.codes[c] + tid;
+		const float2* tw1 = plan.tables;
+		const float2* tw2 = tw1 + R0 * (R1 - 1) + tid;
+		if (tid < NB2)
+#pragma unroll
+			for (int r = 0; r < R2; ++r)
+				acc[tid + r * NB2] = 0.f;
+		const float scale = (p.one_sided ? 2.0f : 1.0f) / static_cast<float>(N);
+		const int stat = p.stat;
+		for (int blk = part; blk < p.k_blocks; blk += plan.split) {
+			// code and twiddle reads stay in the loop: held across it they spill
+			asm volatile("" : "+l"(code), "+l"(tw1), "+l"(tw2));
+			if (tid < NB0) {
+				const float2* x = p.spectra + (static_cast<size_t>(d) * p.k_blocks + blk) * N + tid;
+				float2 v[R0];
+#pragma unroll
+				for (int r = 0; r < RL; ++r)
+					v[r] = __ldg(x + r * NB0);
+#pragma unroll
+				for (int r = 0; r < RL; ++r)
+					v[r] = (HALF || p.one_sided) && tid + r * NB0 > N / 2 ? c2(0.f, 0.f) : cmul(v[r], __ldg(code + r * NB0));
+				if constexpr (RL < R0)
+					DftPruned<R0, true, RL>::run(v);
+				else
+					Dft<R0, true>::run(v);
+#pragma unroll
+				for (int r = 0; r < R0; ++r)
+					first[r] = v[r];
+			}
+			__syncthreads();
+			for (int u = tid; u < NB1; u += kSmallThreads) {  // u = k0 + R0 j1
+				const float2* w = tw1 + u % R0;
+				float2 v[R1];
+#pragma unroll
+				for (int r = 0; r < R1; ++r)
+					v[r] = t[u + r * GS];
+#pragma unroll
+				for (int r = 1; r < R1; ++r)
+					v[r] = cmulc(v[r], __ldg(w + (r - 1) * R0));
+				Dft<R1, true>::run(v);
+#pragma unroll
+				for (int r = 0; r < R1; ++r)
+					t[u + r * GS] = v[r];
+			}
+			__syncthreads();
+			if (tid < NB2) {
+				float2 v[R2];
+#pragma unroll
+				for (int r = 0; r < R2; ++r)
+					v[r] = last[r * R0];
+#pragma unroll
+				for (int r = 1; r < R2; ++r)
+					v[r] = cmulc(v[r], __ldg(tw2 + (r - 1) * NB2));
+				Dft<R2, true>::run(v);
+				float m[R2];
+				stats_of(v, scale, stat, m);
+#pragma unroll
+				for (int r = 0; r < R2; ++r)
+					acc[tid + r * NB2] += m[r];
+			}
+			__syncthreads();  // the next block's pass 0 rewrites the tile
+		}
+		if (plan.split > 1 && !cluster_sum(acc, N, plan.split, part))
+			return;
+		__syncthreads();
+		reduce_cell(acc, N, p.cells + static_cast<size_t>(c) * p.n_doppler + p.d_base + d);
 	}
 
 	template <class K>
@@ -255,11 +430,11 @@ namespace ugsdr_gpu {
 
 	// the launch error, if any, is the runtime's last error
 	template <class K>
-	void launch_inv_small(K kernel, const AcqParams& p, const SmallPlan& plan, int rows, cudaStream_t stream) {
+	void launch_inv_small(K kernel, const AcqParams& p, const SmallPlan& plan, int rows, int smem, cudaStream_t stream) {
 		cudaLaunchConfig_t cfg{};
 		cfg.gridDim = dim3(static_cast<unsigned>(rows) * plan.split);
 		cfg.blockDim = dim3(plan.threads);
-		cfg.dynamicSmemBytes = small_inv_bytes(plan);
+		cfg.dynamicSmemBytes = smem;
 		cfg.stream = stream;
 		cudaLaunchAttribute cluster{};
 		cluster.id = cudaLaunchAttributeClusterDimension;

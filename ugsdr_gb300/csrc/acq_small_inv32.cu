@@ -3,6 +3,7 @@
 
 namespace ugsdr_gpu {
 	void launch_inv_small32(const AcqParams& p, const SmallPlan& plan, int rows, cudaStream_t stream) {
-		launch_inv_small(p.one_sided ? acq_inv_small_kernel<32, true> : acq_inv_small_kernel<32, false>, p, plan, rows, stream);
+		launch_inv_small(p.one_sided ? acq_inv_small_kernel<32, true> : acq_inv_small_kernel<32, false>, p, plan, rows,
+			small_inv_bytes(plan), stream);
 	}
 }
