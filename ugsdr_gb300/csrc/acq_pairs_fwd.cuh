@@ -9,8 +9,10 @@
 // gather reads).  A CTA takes up to four (Doppler, block) items of its columns
 // or rows, so that its tables and twiddle seeds are built once; fewer when the
 // items are too few to fill the SMs (36 items of 50,000 points: 128 -> 121 us a
-// search).
-// Bound: issue and the latency of the loads.
+// search).  Splits of radices up to 25 run at 80 registers a thread (24 warps
+// per SM, not 15): 656 items of 50,000 points and 16 x 41 x 40 more, columns
+// 5.4 -> 4.8 ms, rows 4.6 -> 3.9.
+// Bound: issue (72 % in the columns) and the latency of the loads.
 #pragma once
 
 #include "acq_pairs.cuh"
@@ -35,8 +37,8 @@ namespace ugsdr_gpu {
 	}
 
 	// grid: ceil(items / per) * ceil(N2 / 8)
-	template <int ST>
-	__global__ void __launch_bounds__(kPairThreads, 2) fwd_cols_pair_kernel(const __grid_constant__ BatchedParams p, int items,
+	template <int ST, int MAXR>
+	__global__ void __launch_bounds__(kPairThreads, kPairMinBlocks<MAXR>) fwd_cols_pair_kernel(const __grid_constant__ BatchedParams p, int items,
 		int per) {
 		extern __shared__ __align__(16) unsigned char raw[];
 		__shared__ float lut[80];
@@ -71,7 +73,7 @@ namespace ugsdr_gpu {
 			const uint32_t adder = q.adders[q.d_base + d], fe_adder = q.fe_adder;
 			const int fe_on = q.fe_on;
 			// pass 0: radix a0, sample n2 (j + r a1) + c0 + c (u = j CW + c)
-			with_radix<32>(a0, [&](auto rc) {
+			with_radix<MAXR>(a0, [&](auto rc) {
 				constexpr int R = decltype(rc)::value;
 				constexpr int PAD = (R & 1) ^ 1;
 				const uint32_t dg = static_cast<uint32_t>(n2) * static_cast<uint32_t>(a1);
@@ -110,7 +112,7 @@ namespace ugsdr_gpu {
 			__syncthreads();
 			// pass 1: radix a1, output k1 = j + r a0, times W_N^{(c0 + c) k1}
 			float2* out = p.out + static_cast<size_t>(item) * n + c0;
-			with_radix<32>(a1, [&](auto rc) {
+			with_radix<MAXR>(a1, [&](auto rc) {
 				constexpr int R = decltype(rc)::value;
 				const size_t inc = static_cast<size_t>(a0) * n2;
 				for (int u = threadIdx.x; u < CW * a0; u += blockDim.x) {
@@ -147,14 +149,15 @@ namespace ugsdr_gpu {
 		const int seeds = lay.acc_at + static_cast<int>(sizeof(float2)) * 8 * (p.pair.a0 + 1);
 		const int parts = (p.n2 + 7) / 8, per = pair_items(items, parts, sm_count);
 		const int grid = (items + per - 1) / per * parts;
-		cudaFuncSetAttribute(fwd_cols_pair_kernel<ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem);
-		fwd_cols_pair_kernel<ST><<<grid, pair_fwd_threads(8 * min(p.pair.a0, p.pair.a1)), seeds, stream>>>(p, items, per);
+		auto kernel = max(p.pair.a0, p.pair.a1) <= 25 ? fwd_cols_pair_kernel<ST, 25> : fwd_cols_pair_kernel<ST, 32>;
+		cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem);
+		kernel<<<grid, pair_fwd_threads(8 * min(p.pair.a0, p.pair.a1)), seeds, stream>>>(p, items, per);
 	}
 
 	// grid: ceil(items / per) * ceil(N1 / rw); spectra elements k2 <
 	// row_keep (0: all) of each row stored
-	template <class = void>
-	__global__ void __launch_bounds__(kPairThreads, 2) fwd_rows_pair_kernel(const __grid_constant__ BatchedParams p, int items,
+	template <int MAXR>
+	__global__ void __launch_bounds__(kPairThreads, kPairMinBlocks<MAXR>) fwd_rows_pair_kernel(const __grid_constant__ BatchedParams p, int items,
 		int per) {
 		extern __shared__ __align__(16) unsigned char raw[];
 		const int b0 = p.pair.b0, b1 = p.pair.b1, n1 = p.n1, n2 = p.n2;
@@ -175,7 +178,7 @@ namespace ugsdr_gpu {
 		const int it1 = min(items, (group + 1) * per);
 		for (int item = group * per; item < it1; ++item) {
 			float2* rows = p.out + static_cast<size_t>(item) * p.base.n + static_cast<size_t>(r0) * n2;
-			with_radix<32>(b0, [&](auto rc) {
+			with_radix<MAXR>(b0, [&](auto rc) {
 				constexpr int R = decltype(rc)::value;
 				constexpr int PAD = (R & 1) ^ 1;
 				for (int u = threadIdx.x; u < rw * b1; u += blockDim.x) {
@@ -193,7 +196,7 @@ namespace ugsdr_gpu {
 				}
 			});
 			__syncthreads();  // the CTA's rows are read: pass 1 may write over them
-			with_radix<32>(b1, [&](auto rc) {
+			with_radix<MAXR>(b1, [&](auto rc) {
 				constexpr int R = decltype(rc)::value;
 				const int stride = b0 + lay.pad;
 				for (int u = threadIdx.x; u < rw * b0; u += blockDim.x) {
