@@ -15,6 +15,7 @@ namespace ugsdr_gpu {
 		auto launch = [&](auto kernel) {
 			UG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem));
 			kernel<<<grid, s.col_threads, lay.bytes, stream>>>(p);
+			UG_CUDA(cudaGetLastError());
 		};
 		if (std::max(s.a0, s.a1) <= 25)
 			p.base.stat ? launch(inv_cols_pair_kernel<CW, 25, 1>) : launch(inv_cols_pair_kernel<CW, 25, 0>);

@@ -12,6 +12,7 @@ namespace ugsdr_gpu {
 		auto launch = [&](auto kernel) {
 			UG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem));
 			kernel<<<grid, s.row_threads, lay.bytes, stream>>>(p);
+			UG_CUDA(cudaGetLastError());
 		};
 		if (std::max(s.b0, s.b1) <= 25)
 			half ? launch(inv_rows_pair_kernel<25, true>) : launch(inv_rows_pair_kernel<25, false>);
