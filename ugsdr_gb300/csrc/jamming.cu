@@ -218,7 +218,8 @@ namespace ugsdr_gpu {
 		struct DetectParams {
 			const float2* x;       // samples; column c starts at 32 c
 			int cols;
-			int batches;           // of 32 columns
+			int per_octet;         // columns per octet of lanes and batch
+			int batches;           // of 4 per_octet columns
 			const float* window;   // 128 Hann coefficients
 			const float2* tw;      // W_128^m, m < 128
 			DetectScratch det;
@@ -313,9 +314,10 @@ namespace ugsdr_gpu {
 		}
 
 		// JammingDetector's STFT and per-column candidates: a warp takes batches of
-		// 32 consecutive columns (grid-stride), each octet of lanes eight of them in
-		// a row — a column's samples are the previous one's moved by 32, so only 32
-		// are loaded per column — then each lane one column's candidates.  Bound:
+		// 4 per_octet consecutive columns (grid-stride), each octet of lanes
+		// per_octet (eight, fewer for short signals) of them in a row — a column's
+		// samples are the previous one's moved by 32, so only 32 are loaded per
+		// column — then each lane one column's candidates.  Bound:
 		// issue, and shared memory for the warps in flight.
 		__global__ void __launch_bounds__(kDetectThreads) detect_kernel(DetectParams p) {
 			extern __shared__ __align__(16) unsigned char raw[];
@@ -338,7 +340,7 @@ namespace ugsdr_gpu {
 				win[j] = p.window[fft.l + 8 * j];
 			const int warps = gridDim.x * (blockDim.x >> 5);
 			for (int batch = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); batch < p.batches; batch += warps) {
-				const int c0 = batch * 32 + octet * 8;  // the octet's first column
+				const int c0 = (batch * 4 + octet) * p.per_octet;  // the octet's first column
 				// samples of the last column on (clamped: columns past the end repeat it)
 				const float2* x = p.x + static_cast<size_t>(min(c0, p.cols - 1)) * 32 + fft.l;
 				float2 smp[16];
@@ -346,7 +348,7 @@ namespace ugsdr_gpu {
 				for (int j = 0; j < 12; ++j)
 					smp[j + 4] = x[8 * j];
 #pragma unroll 1
-				for (int i = 0; i < 8; ++i) {
+				for (int i = 0; i < p.per_octet; ++i) {
 #pragma unroll
 					for (int j = 0; j < 12; ++j)
 						smp[j] = smp[j + 4];
@@ -360,14 +362,14 @@ namespace ugsdr_gpu {
 					for (int j = 0; j < 16; ++j)  // vec * complex(window, 0) (stft.hpp:55-56): both parts scaled
 						v[j] = c2(__fmul_rn(smp[j].x, win[j]), __fmul_rn(smp[j].y, win[j]));
 					fft.forward(v);
-					float* m = mags + (octet * 8 + i) * kMagStride + fft.l;
+					float* m = mags + (octet * p.per_octet + i) * kMagStride + fft.l;
 #pragma unroll
 					for (int j = 0; j < 16; ++j)
 						m[8 * j] = __fsqrt_rn(v[j].x * v[j].x + v[j].y * v[j].y);
 				}
 				__syncwarp();
-				const int col = batch * 32 + lane;
-				if (col < p.cols)
+				const int col = batch * 4 * p.per_octet + lane;
+				if (lane < 4 * p.per_octet && col < p.cols)
 					detect_column(mags + lane * kMagStride, groups + lane * 17, p.det, static_cast<size_t>(col), static_cast<size_t>(p.cols),
 						s_hist, &s_total);
 				__syncwarp();  // the next batch writes the magnitudes
@@ -678,11 +680,12 @@ namespace ugsdr_gpu {
 			p.n = n;
 			p.cols = static_cast<int>(stft_columns(n, kDetectWindow, kDetectOverlap));
 			// runs of up to 64 slots (each walks three more columns), of the length
-			// that makes whole waves of the CTAs three of which share an SM
+			// that makes whole waves of the CTAs three of which share an SM, two
+			// slots at least
 			const long long slots = static_cast<long long>((n + 31) / 32);
 			const long long wave = static_cast<long long>(ctx->sm_count) * 3 * (kWidebandThreads / 8);  // octets
 			const long long waves = (slots + 64 * wave - 1) / (64 * wave);
-			p.slots_per_octet = static_cast<int>(std::max<long long>(8, (slots + waves * wave - 1) / (waves * wave)));
+			p.slots_per_octet = static_cast<int>(std::max<long long>(2, (slots + waves * wave - 1) / (waves * wave)));
 			p.window = hann_window(ctx, kDetectWindow);
 			p.tw = get_plan(ctx, kDetectWindow).tw;
 			p.out = out;
@@ -838,7 +841,12 @@ namespace ugsdr_gpu {
 			DetectParams dp{};
 			dp.x = x;
 			dp.cols = static_cast<int>(cols);
-			dp.batches = static_cast<int>((cols + 31) / 32);
+			// fewer columns in a row until the warps fill the SMs (eight per SM):
+			// 4,474 columns 17 us by eight in a row, 9 one at a time
+			dp.per_octet = 8;
+			while (dp.per_octet > 1 && cols < static_cast<size_t>(4 * dp.per_octet) * 8 * ctx->sm_count)
+				dp.per_octet /= 2;
+			dp.batches = static_cast<int>((cols + 4 * dp.per_octet - 1) / (4 * dp.per_octet));
 			dp.window = hann_window(ctx, kDetectWindow);
 			dp.tw = get_plan(ctx, kDetectWindow).tw;
 			dp.det = d;
