@@ -841,10 +841,10 @@ namespace ugsdr_gpu {
 			DetectParams dp{};
 			dp.x = x;
 			dp.cols = static_cast<int>(cols);
-			// fewer columns in a row until the warps fill the SMs (eight per SM):
+			// fewer columns in a row as long as one wave of warps (eight per SM) holds them:
 			// 4,474 columns 17 us by eight in a row, 9 one at a time
 			dp.per_octet = 8;
-			while (dp.per_octet > 1 && cols < static_cast<size_t>(4 * dp.per_octet) * 8 * ctx->sm_count)
+			while (dp.per_octet > 1 && cols <= static_cast<size_t>(2 * dp.per_octet) * 8 * ctx->sm_count)
 				dp.per_octet /= 2;
 			dp.batches = static_cast<int>((cols + 4 * dp.per_octet - 1) / (4 * dp.per_octet));
 			dp.window = hann_window(ctx, kDetectWindow);
