@@ -128,7 +128,7 @@ namespace ugsdr_gpu {
 		const float sc = STAT ? s * s : s;
 		const int n2g = chunk * P::CW + warp * P::CPW + c1;
 		MaxIdx best{-1.0f, 0xFFFFFFFFu};
-		float sum = 0.f, sq = 0.f;
+		float sum = 0.f;
 		if (n2g < n2) {
 #pragma unroll
 			for (int r = 0; r < P::R1; ++r) {  // n1 increases with r: strict > keeps the first maximum
@@ -138,10 +138,14 @@ namespace ugsdr_gpu {
 					best.i = static_cast<uint32_t>(n2) * static_cast<uint32_t>(j1 + r * P::R0) + static_cast<uint32_t>(n2g);
 				}
 				sum += v;
-				sq += v * v;
 			}
 		}
-		double dsum = sum, dsq = sq;
+		const Moments own = moments(n2g < n2 ? P::R1 : 0, sum, [&](auto&& add) {
+#pragma unroll
+			for (int r = 0; r < P::R1; ++r)
+				add(acc[r] * sc);
+		});
+		double dsum = own.sum, dsq = own.sq;
 		for (int o = 16; o > 0; o >>= 1) {
 			const MaxIdx other{__shfl_down_sync(0xffffffffu, best.v, o), __shfl_down_sync(0xffffffffu, best.i, o)};
 			best = better(best, other);

