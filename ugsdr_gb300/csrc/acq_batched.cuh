@@ -929,23 +929,20 @@ namespace ugsdr_gpu {
 			return;
 		// chunk partial: first max (lowest natural index on ties), sum, sum of squares (moments)
 		MaxIdx best{-1.0f, 0xFFFFFFFFu};
-		float sum = 0.f;
-		int count = 0;
+		auto value = [&](int e) {
+			const int f = div_fft_n<F1>(e, inv_n1);
+			return acc[f * ld + e - f * n1];
+		};
+		const int e_last = cw * n1 - 1;
+		Moments own(value(min(static_cast<int>(threadIdx.x), e_last)), value(min(static_cast<int>(threadIdx.x + blockDim.x), e_last)));
 		for (int e = threadIdx.x; e < cw * n1; e += blockDim.x) {
 			const int f = div_fft_n<F1>(e, inv_n1), i1 = e - f * n1;
 			const float v = acc[f * ld + i1];
 			const MaxIdx cand{v, static_cast<uint32_t>(n2) * i1 + c0 + f};
 			best = better(best, cand);
-			sum += v;
-			++count;
+			own.add(v);
 		}
-		const Moments own = moments(count, sum, [&](auto&& add) {
-			for (int e = threadIdx.x; e < cw * n1; e += blockDim.x) {
-				const int f = div_fft_n<F1>(e, inv_n1);
-				add(acc[f * ld + e - f * n1]);
-			}
-		});
-		double dsum = own.sum, dsq = own.sq;
+		double dsum = own.sum(), dsq = own.squares();
 		for (int o = 16; o > 0; o >>= 1) {
 			const MaxIdx other{__shfl_down_sync(0xffffffffu, best.v, o), __shfl_down_sync(0xffffffffu, best.i, o)};
 			best = better(best, other);

@@ -128,7 +128,7 @@ namespace ugsdr_gpu {
 		const float sc = STAT ? s * s : s;
 		const int n2g = chunk * P::CW + warp * P::CPW + c1;
 		MaxIdx best{-1.0f, 0xFFFFFFFFu};
-		float sum = 0.f;
+		Moments own(acc[0] * sc, acc[1] * sc);
 		if (n2g < n2) {
 #pragma unroll
 			for (int r = 0; r < P::R1; ++r) {  // n1 increases with r: strict > keeps the first maximum
@@ -137,15 +137,10 @@ namespace ugsdr_gpu {
 					best.v = v;
 					best.i = static_cast<uint32_t>(n2) * static_cast<uint32_t>(j1 + r * P::R0) + static_cast<uint32_t>(n2g);
 				}
-				sum += v;
+				own.add(v);
 			}
 		}
-		const Moments own = moments(n2g < n2 ? P::R1 : 0, sum, [&](auto&& add) {
-#pragma unroll
-			for (int r = 0; r < P::R1; ++r)
-				add(acc[r] * sc);
-		});
-		double dsum = own.sum, dsq = own.sq;
+		double dsum = own.sum(), dsq = own.squares();
 		for (int o = 16; o > 0; o >>= 1) {
 			const MaxIdx other{__shfl_down_sync(0xffffffffu, best.v, o), __shfl_down_sync(0xffffffffu, best.i, o)};
 			best = better(best, other);

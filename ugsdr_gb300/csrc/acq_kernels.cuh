@@ -246,30 +246,31 @@ namespace ugsdr_gpu {
 		return a;
 	}
 
-	// Sum and sum of squares, in double, of a thread's n values each(f) hands to
-	// f in turn, `sum` being their float sum.  Squares of magnitudes summed over
-	// K blocks cancel like (mean / sigma)^2 = 3.7 K in the variance, so floats
-	// sum only deviations from the thread's own mean a: sum v = n a + d and
-	// sum v^2 = sum (v - a)^2 + 2 a d + n a^2 hold for any a.  At 10,230 points
-	// and K = 1,000 sigma is then within 4e-7 of 64 bits; float squares left
-	// 1.2e-5.  Sums beyond float's range stay what they are.
+	// Sum and sum of squares, in double, of a thread's values.  Squares of
+	// magnitudes summed over K blocks cancel like (mean / sigma)^2 = 3.7 K in the
+	// variance, so floats sum only the deviations from a value a of the thread's
+	// own: sum v = n a + d and sum v^2 = sum (v - a)^2 + 2 a d + n a^2 hold for
+	// any a, and the smaller of two values is no correlation peak.  At 10,230
+	// points and K = 1,000 sigma is then within 4e-7 of 64 bits; float squares
+	// left 1.2e-5.
 	struct Moments {
-		double sum, sq;
-	};
-	template <class Each>
-	__device__ __forceinline__ Moments moments(int n, float sum, Each&& each) {
-		if (n == 0 || !(fabsf(sum) <= 3.4028234e38f))
-			return Moments{sum, sum};
-		const float a = sum / static_cast<float>(n);
-		float d = 0.f, m2 = 0.f;
-		each([&](float v) {
+		float a, d, m2;
+		int n;
+		__device__ __forceinline__ Moments(float v0, float v1) : a(fminf(v0, v1)), d(0.f), m2(0.f), n(0) {
+			if (!(a <= 3.4028234e38f))
+				a = 0.f;  // sums beyond float's range stay what they are
+		}
+		__device__ __forceinline__ void add(float v) {
 			const float e = v - a;
 			d += e;
 			m2 = fmaf(e, e, m2);
-		});
-		const double da = a, dd = d, dn = n;
-		return Moments{dn * da + dd, m2 + da * (2.0 * dd + dn * da)};
-	}
+			++n;
+		}
+		__device__ __forceinline__ double sum() const { return static_cast<double>(n) * a + d; }
+		__device__ __forceinline__ double squares() const {
+			return m2 + static_cast<double>(a) * (2.0 * d + static_cast<double>(n) * a);
+		}
+	};
 
 	// reduces acc[0..m) into one cell (first maximum, mean, unbiased std)
 	static __device__ void reduce_cell(const float* acc, int m, AcqCellDev* out) {

@@ -270,8 +270,9 @@ namespace ugsdr_gpu {
 		const float s = (q.one_sided ? 2.0f : 1.0f) / static_cast<float>(q.n);
 		const float sc = STAT ? s * s : s;
 		MaxIdx best{-1.0f, 0xFFFFFFFFu};
-		float sum = 0.f;
-		int count = 0;
+		const float* const first = acc + threadIdx.x * lay.accs;
+		const bool any = threadIdx.x < CW * a0;
+		Moments own(any ? first[0] * sc : 0.f, any ? first[1] * sc : 0.f);
 		for (int u = threadIdx.x; u < CW * a0; u += blockDim.x) {
 			const int j = u / CW, n2g = chunk * CW + u % CW;
 			if (n2g >= n2)
@@ -279,17 +280,10 @@ namespace ugsdr_gpu {
 			for (int r = 0; r < a1; ++r) {
 				const float v = acc[u * lay.accs + r] * sc;
 				best = better(best, MaxIdx{v, static_cast<uint32_t>(n2) * static_cast<uint32_t>(j + r * a0) + static_cast<uint32_t>(n2g)});
-				sum += v;
+				own.add(v);
 			}
-			count += a1;
 		}
-		const Moments own = moments(count, sum, [&](auto&& add) {
-			for (int u = threadIdx.x; u < CW * a0; u += blockDim.x)
-				if (chunk * CW + u % CW < n2)
-					for (int r = 0; r < a1; ++r)
-						add(acc[u * lay.accs + r] * sc);
-		});
-		double dsum = own.sum, dsq = own.sq;
+		double dsum = own.sum(), dsq = own.squares();
 		auto warp_reduce = [&] {
 			for (int o = 16; o > 0; o >>= 1) {
 				const MaxIdx other{__shfl_down_sync(0xffffffffu, best.v, o), __shfl_down_sync(0xffffffffu, best.i, o)};
