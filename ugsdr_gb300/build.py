@@ -25,7 +25,8 @@ ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 NVCC_FLAGS = ["-std=c++17", "--expt-relaxed-constexpr", "-O3", "-lineinfo", "-Xcompiler", "-fPIC",
               "-Xcompiler", "-ffp-contract=off", "-I", str(ROOT / "include")]
 SOURCES = ["acq.cu", "acq_pairs_rows.cu", "acq_pairs_cols4.cu", "acq_pairs_cols8.cu", "acq_small_fwd_8bit.cu", "acq_small_fwd_wide.cu",
-           "acq_small_inv25.cu", "acq_small_inv32.cu",
+           "acq_small_inv25.cu", "acq_small_inv25_cluster.cu", "acq_small_inv32.cu", "acq_small_inv32_cluster.cu",
+           "acq_small_two_sided.cu", "acq_small_two_sided_cluster.cu",
            "acq_pairs_fwd_cf32.cu", "acq_pairs_fwd_ci8.cu", "acq_pairs_fwd_ci16.cu", "acq_pairs_fwd_ri8.cu", "acq_pairs_fwd_rows.cu",
            "ops.cu", "ctx.cu", "track.cu", "serve.cpp", "codes.cpp", "noalloc.cu", "refine.cpp", "jamming.cu", "observables.cu", "tc_dft.cu"]
 

@@ -1013,28 +1013,36 @@ namespace ugsdr_gpu {
 		}
 
 		// CTAs per row (a cluster of eight at most): the cheapest of rows x split
-		// CTAs, each with its share of the K blocks and two blocks' worth of
-		// setup and summing.  An SM holds `cap` CTAs and runs 512 / threads of
-		// them at the pace of one; beyond `cap`, the mean of whole rounds and of
-		// a steady flow with three quarters of a CTA for its tail; the most
-		// CTAs among equals.  Fitted to 8
-		// sizes of 1,023 to 5,000 points, 21 to 2,592 rows, K 2 to 20: the
-		// rule's pick is within 10 % of the best split at most shapes (168 rows x
-		// 4 of 5,000 points: 36 us unsplit, 49 by two; 84 x 10: 57, 45, 38 by three).
-		int wave_split(ugsdr_ctx* ctx, int rows, int k_blocks, int threads, int cap) {
-			const double free = 512.0 / threads;
+		// CTAs, each with its share of the K blocks, three blocks' worth of setup and
+		// reduction and half a block's for each further round of a cluster's sums.
+		// An SM holds `cap` CTAs (shared memory, and most_ctas by registers) and
+		// runs 512 / threads of them at the pace of one; beyond `cap`, the mean of
+		// whole rounds and of a steady flow with three quarters of a CTA for its
+		// tail; the most CTAs among equals.  Fitted to 8 sizes of 500 to 5,456
+		// points, 1 to 672 rows, K 2 to 40, every split: the rule's pick is 2.2 %
+		// slower than the best split on average (one row x 40 of 5,000 points: 190
+		// us unsplit, 51 by eight; 84 x 10: 57, 51 by three, 70 by eight; 672 x 20:
+		// 330, 493 by two).
+		int wave_split(ugsdr_ctx* ctx, SmallPlan plan, int rows, int k_blocks, int most_ctas) {
+			const double free = 512.0 / plan.threads;
 			auto round = [&](int ctas) { return ctas ? std::max(1.0, ctas / free) : 0.0; };
 			int best = 1;
 			double best_cost = 1e300;
 			for (int s = 1; s <= std::min(8, k_blocks); ++s) {
+				plan.split = s;
+				const int bytes = small_inv_bytes(plan) + small_cluster_bytes(plan);
+				if (bytes > kSmallSmem)
+					continue;
+				const int cap = std::max(1, std::min((kSmallSmem + 1024) / (bytes + 1024), most_ctas));
 				const int share = (k_blocks + s - 1) / s;
 				const double mean = static_cast<double>(rows) * s / ctx->sm_count;
 				const int most = static_cast<int>(std::ceil(mean));
 				double load = most / cap * round(cap) + round(most % cap);
 				if (most > cap)
 					load = 0.5 * (load + (mean + 0.75) / free);
-				if (load * (share + 2) <= best_cost) {
-					best_cost = load * (share + 2);
+				const double cost = load * (share + 3 + (s > 1 ? 0.5 * (share - 1) : 0.0));
+				if (cost <= best_cost) {
+					best_cost = cost;
 					best = s;
 				}
 			}
@@ -1071,9 +1079,7 @@ namespace ugsdr_gpu {
 			for (int t = 64; t <= kSmallThreads; t += 32)
 				if (cost(t) <= 1.1 * best)
 					p.threads = t;
-			// resident CTAs: shared memory, and 128 registers a thread
-			const int cap = std::min(kSmallSmem / (small_inv_bytes(p) + 1024), 512 / p.threads);
-			p.split = wave_split(ctx, rows, k_blocks, p.threads, std::max(1, cap));
+			p.split = wave_split(ctx, p, rows, k_blocks, std::max(1, 512 / p.threads));  // 128 registers a thread
 			return p;
 		}
 
@@ -1122,7 +1128,7 @@ namespace ugsdr_gpu {
 			plan.radix[2] = 16;
 			plan.tables = pass_tables(ctx, plan);
 			plan.threads = kSmallThreads;
-			plan.split = wave_split(ctx, nd * n_codes, k, kSmallThreads, 3);
+			plan.split = wave_split(ctx, plan, nd * n_codes, k, 3);
 			// one-sided spectra: pass 0 reads only the lower half of Z
 			launch_inv_4000(p, plan, p.one_sided && !std::getenv("UGSDR_NO_PRUNE"), nd * n_codes, ctx->stream);
 			note_launch(ctx);

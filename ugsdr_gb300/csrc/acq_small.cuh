@@ -7,8 +7,8 @@
 // from a per-size table in the order [r - 1][k] (coalesced over the lanes'
 // consecutive k; L1).
 // acq_inv_small_kernel splits the K blocks of a (code, Doppler) row over the
-// CTAs of a cluster when the rows alone leave SMs idle; the first CTA adds the
-// others' accumulators through distributed shared memory.
+// CTAs of a cluster when the rows alone leave SMs idle; the CTAs add their
+// magnitudes in block order through distributed shared memory.
 // Bound: issue and the barriers between the passes.
 #pragma once
 
@@ -48,9 +48,18 @@ namespace ugsdr_gpu {
 	inline int small_tiles_bytes(const SmallPlan& plan) {
 		return static_cast<int>(sizeof(float2)) * (small_tile(plan) + (plan.n_pass > 2 ? plan.n : 0));
 	}
+	// accumulators, 16-byte pieces of them
+	UG_HD constexpr int small_accs(int n) { return (n + 3) / 4 * 4; }
 	inline int small_inv_bytes(const SmallPlan& plan) {
-		return static_cast<int>(sizeof(float2)) * ((plan.n + 1) / 2) + (plan.n_pass == 3
-			? static_cast<int>(sizeof(float2)) * InPlace(plan.radix[0], plan.radix[1], plan.radix[2]).elems : small_tiles_bytes(plan));
+		const int tile = plan.n_pass == 3
+			? static_cast<int>(sizeof(float2)) * InPlace(plan.radix[0], plan.radix[1], plan.radix[2]).elems : small_tiles_bytes(plan);
+		return static_cast<int>(sizeof(float)) * small_accs(plan.n) + (tile + 15) / 16 * 16;
+	}
+	// beyond those, bytes: a cluster CTA's second buffer of magnitudes and its
+	// share of the running sums
+	UG_HD int small_cluster_bytes(const SmallPlan& plan) {
+		const int step = 4 * plan.split * plan.threads;
+		return plan.split > 1 ? static_cast<int>(sizeof(float)) * (small_accs(plan.n) + (plan.n + step - 1) / step * 4 * plan.threads) : 0;
 	}
 	// every kernel's limit, set to it always: a context with smaller blocks
 	// never lowers it under another's launch
@@ -179,33 +188,44 @@ namespace ugsdr_gpu {
 		});
 	}
 
-	// Distributed shared memory: adds the n accumulators of a cluster's `split`
-	// CTAs into the first one's, in order; true in that CTA.  Every CTA sums its
-	// share of the n (a CTA alone reading the others' waits a round trip per
-	// element and CTA: half the kernel's time at 168 rows of 2,500 points).
-	__device__ __forceinline__ bool cluster_sum(float* acc, int n, int split, int part) {
-		asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-		const uint32_t mine = static_cast<uint32_t>(__cvta_generic_to_shared(acc));
+	__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+	__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+
+	// Adds a round of a cluster's CTAs, the first `live` of which hold a block's n
+	// magnitudes in mag, in block order to the running sums, of which every CTA
+	// keeps its share in tot (a CTA alone reading the others' waits a round trip
+	// per element and CTA: half the kernel's time at 168 rows of 2,500 points).
+	// A cell's sum is so the one a lone CTA makes of its blocks, whatever the
+	// split, and the split may follow the rows of a launch.  The last round
+	// leaves the sums in the first CTA's mag.  Between a wait for the round's
+	// magnitudes and an arrival.
+	__device__ __forceinline__ void cluster_add(float* mag, float* tot, int n, int split, int part, int live, bool first, bool last) {
+		const uint32_t mine = static_cast<uint32_t>(__cvta_generic_to_shared(mag));
 		uint32_t at[8];
 #pragma unroll
 		for (int o = 0; o < 8; ++o)
 			if (o < split)
 				asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at[o]) : "r"(mine), "r"(o));
-		for (int i = part * blockDim.x + threadIdx.x; i < n; i += split * blockDim.x) {
-			float v[8];
+		// four sums a thread: a round trip per 4 x split x threads of them
+		float4* const sums = reinterpret_cast<float4*>(tot);
+		for (int i = part * blockDim.x + threadIdx.x, j = threadIdx.x; i < (n + 3) / 4; i += split * blockDim.x, j += blockDim.x) {
+			float4 v[8];
 #pragma unroll
 			for (int o = 0; o < 8; ++o)
-				if (o < split)
-					asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v[o]) : "r"(at[o] + 4u * i) : "memory");
-			float s = v[0];
+				if (o < live)
+					asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+						: "=f"(v[o].x), "=f"(v[o].y), "=f"(v[o].z), "=f"(v[o].w) : "r"(at[o] + 16u * i) : "memory");
+			float4 s = first ? make_float4(0.f, 0.f, 0.f, 0.f) : sums[j];
 #pragma unroll
-			for (int o = 1; o < 8; ++o)
-				if (o < split)
-					s += v[o];
-			asm volatile("st.shared::cluster.f32 [%0], %1;" :: "r"(at[0] + 4u * i), "f"(s) : "memory");
+			for (int o = 0; o < 8; ++o)
+				if (o < live)
+					s = make_float4(s.x + v[o].x, s.y + v[o].y, s.z + v[o].z, s.w + v[o].w);
+			if (last)
+				asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};"
+					:: "r"(at[0] + 16u * i), "f"(s.x), "f"(s.y), "f"(s.z), "f"(s.w) : "memory");
+			else
+				sums[j] = s;
 		}
-		asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-		return part == 0;
 	}
 
 	// grid: (rows x split) CTAs in clusters of `split`; unfolded rows (m == N).
@@ -216,16 +236,21 @@ namespace ugsdr_gpu {
 	// 3,000 points 139 us against 110.
 	// HALF: one-sided spectra (Z is zero above N / 2: pass 0 reads R / 2 + 1 of
 	// its R inputs)
-	template <int MAXR, bool HALF>
+	// CLUSTER: split > 1 (apart, as its sums cost the lone CTAs' kernel registers:
+	// 255 -> 267 us for 32 codes x 21 bins x 20 blocks of 2,046 points)
+	template <int MAXR, bool HALF, bool CLUSTER>
 	__global__ void __launch_bounds__(kSmallThreads, HALF ? 2 : 1) acq_inv_small_kernel(const __grid_constant__ AcqParams p,
-		const __grid_constant__ SmallPlan plan) {
-		extern __shared__ float2 smem[];
+		const __grid_constant__ SmallPlan plan, int mag_at) {
+		extern __shared__ __align__(16) float2 smem[];
 		const int n = plan.n;
 		float* const acc = reinterpret_cast<float*>(smem);
-		float2* const a = smem + (n + 1) / 2;
+		// (the same offset in a lone CTA spilled 500 bytes more at radix 31, 4 - 14 %)
+		float2* const a = smem + (CLUSTER ? small_accs(n) / 2 : (n + 1) / 2);
 		float2* const b = a + small_tile(plan);
-		const int row = blockIdx.x / plan.split;
-		const int part = blockIdx.x - row * plan.split;
+		float* const mag = acc + mag_at;  // a cluster CTA's magnitudes: here and in acc by turns
+		const int split = CLUSTER ? plan.split : 1;
+		const int row = blockIdx.x / split;
+		const int part = blockIdx.x - row * split;
 		const int c = row % p.n_codes;
 		const int d = row / p.n_codes;
 		const float2* code = p.codes[c];
@@ -233,6 +258,7 @@ namespace ugsdr_gpu {
 			acc[i] = 0.f;
 		const float scale = (p.one_sided ? 2.0f : 1.0f) / static_cast<float>(n);
 		const int stat = p.stat;
+		constexpr bool alone = !CLUSTER;
 		// the last pass reads the tile that the next block's first pass rewrites
 		// unless a middle pass (and its barrier) lies between
 		const bool fence = (plan.n_pass & 1) == 0;
@@ -240,7 +266,22 @@ namespace ugsdr_gpu {
 		const int r0 = plan.radix[0], r1 = plan.radix[1], r2 = three ? plan.radix[2] : 1;
 		const InPlace ip(r0, r1, r2);
 		const float inv_r0 = 1.0f / static_cast<float>(r0), inv_r2 = 1.0f / static_cast<float>(r2);
-		for (int blk = part; blk < p.k_blocks; blk += plan.split) {
+		// A cluster's round of blocks is added while the next one's are on their
+		// way, before their magnitudes are written: whoever waits for a round's
+		// has added the one before it, so two buffers do
+		bool odd = true;
+		auto add_round = [&](int blk0, bool last) {
+			cluster_wait();
+			cluster_add(odd ? mag : acc, mag + small_accs(n), n, split, part, min(split, p.k_blocks - blk0), blk0 == 0, last);
+		};
+		for (int blk0 = 0; blk0 < p.k_blocks; blk0 += split) {
+			const int blk = blk0 + part;
+			if (CLUSTER && blk >= p.k_blocks) {  // a last round of fewer blocks than CTAs
+				add_round(blk0 - split, false);
+				odd = !odd;
+				cluster_arrive();
+				break;
+			}
 			const float2* x = p.spectra + (static_cast<size_t>(d) * p.k_blocks + blk) * n;
 			with_radix<MAXR>(plan.radix[0], [&](auto rc) {
 				constexpr int R = decltype(rc)::value;
@@ -288,6 +329,10 @@ namespace ugsdr_gpu {
 					}
 				});
 				__syncthreads();
+				if (!alone && blk0)
+					add_round(blk0 - split, false);
+				odd = !odd;
+				float* const to = odd ? mag : acc;
 				with_radix<MAXR>(r2, [&](auto rc) {
 					constexpr int R = decltype(rc)::value;
 					const int ns = r0 * r1;
@@ -305,29 +350,56 @@ namespace ugsdr_gpu {
 						Dft<R, true>::run(v);
 						float m[R];
 						stats_of(v, scale, stat, m);
+						if constexpr (alone) {
 #pragma unroll
-						for (int r = 0; r < R; ++r)
-							acc[u + r * ns] += m[r];
+							for (int r = 0; r < R; ++r)
+								acc[u + r * ns] += m[r];
+						}
+						else {
+#pragma unroll
+							for (int r = 0; r < R; ++r)
+								to[u + r * ns] = m[r];
+						}
 					}
 				});
+				if (!alone)
+					cluster_arrive();
 				__syncthreads();  // the next block's pass 0 rewrites the tile
 				continue;
 			}
+			if (!alone && blk0)
+				add_round(blk0 - split, false);
+			odd = !odd;
+			float* const to = odd ? mag : acc;
 			small_passes<MAXR, true>(a, b, plan, [&](int u, int ns, auto& v, auto rc) {
 				constexpr int R = decltype(rc)::value;
 				float m[R];
 				stats_of(v, scale, stat, m);
+				if constexpr (alone) {
 #pragma unroll
-				for (int r = 0; r < R; ++r)
-					acc[u + r * ns] += m[r];
+					for (int r = 0; r < R; ++r)
+						acc[u + r * ns] += m[r];
+				}
+				else {
+#pragma unroll
+					for (int r = 0; r < R; ++r)
+						to[u + r * ns] = m[r];
+				}
 			});
+			if (!alone)
+				cluster_arrive();
 			if (fence)
 				__syncthreads();
 		}
-		if (plan.split > 1 && !cluster_sum(acc, n, plan.split, part))
-			return;
+		if (!alone) {
+			add_round((p.k_blocks - 1) / split * split, true);
+			cluster_arrive();
+			cluster_wait();
+			if (part != 0)
+				return;
+		}
 		__syncthreads();
-		reduce_cell(acc, n, p.cells + static_cast<size_t>(c) * p.n_doppler + p.d_base + d);
+		reduce_cell(alone || !odd ? acc : mag, n, p.cells + static_cast<size_t>(c) * p.n_doppler + p.d_base + d);
 	}
 
 	// The same for N = R0 R1 R2 with every pass compiled in.  At 4,000 points
@@ -335,23 +407,26 @@ namespace ugsdr_gpu {
 	// staged twiddle table (112 KB) left two: 672 rows x 10 blocks 128 -> 90 us.
 	// Bound: the L1 / shared-memory data pipe (60 %), issue (51 %) and the
 	// barriers between the passes.
-	template <int R0, int R1, int R2, bool HALF>
+	template <int R0, int R1, int R2, bool HALF, bool CLUSTER>
 	__global__ void __launch_bounds__(kSmallThreads, 3) acq_inv_three_kernel(const __grid_constant__ AcqParams p,
-		const __grid_constant__ SmallPlan plan) {
+		const __grid_constant__ SmallPlan plan, int mag_at) {
 		constexpr int N = R0 * R1 * R2, NB0 = N / R0, NB1 = N / R1, NB2 = N / R2;
 		static_assert(R0 % 2 == 1, "rows of R0 elements: the middle pass's u runs along them");
 		static_assert(NB0 <= kSmallThreads && NB1 <= 2 * kSmallThreads && NB2 <= kSmallThreads, "butterflies per thread");
 		constexpr int RL = HALF ? R0 / 2 + 1 : R0;
 		constexpr InPlace ip(R0, R1, R2);
 		constexpr int GS = ip.group;
-		extern __shared__ float2 smem[];
+		extern __shared__ __align__(16) float2 smem[];
 		float2* const t = smem;
+		static_assert(ip.elems % 2 == 0, "16-byte aligned accumulators");
 		float* const acc = reinterpret_cast<float*>(smem + ip.elems);
+		float* const mag = reinterpret_cast<float*>(smem) + mag_at;  // a cluster CTA's magnitudes: here and in acc by turns
 		const int tid = threadIdx.x;
 		float2* const first = t + tid * R0 + tid / R2 * ip.pad;
 		const float2* const last = t + tid / R0 * GS + tid % R0;
-		const int row = blockIdx.x / plan.split;
-		const int part = blockIdx.x - row * plan.split;
+		const int split = CLUSTER ? plan.split : 1;
+		const int row = blockIdx.x / split;
+		const int part = blockIdx.x - row * split;
 		const int c = row % p.n_codes;
 		const int d = row / p.n_codes;
 		const float2* code = p.codes[c] + tid;
@@ -363,10 +438,18 @@ namespace ugsdr_gpu {
 				acc[tid + r * NB2] = 0.f;
 		const float scale = (p.one_sided ? 2.0f : 1.0f) / static_cast<float>(N);
 		const int stat = p.stat;
-		for (int blk = part; blk < p.k_blocks; blk += plan.split) {
+		constexpr bool alone = !CLUSTER;
+		bool odd = true;
+		auto add_round = [&](int blk0, bool last) {  // as in acq_inv_small_kernel
+			cluster_wait();
+			cluster_add(odd ? mag : acc, mag + small_accs(N), N, split, part, min(split, p.k_blocks - blk0), blk0 == 0, last);
+		};
+		for (int blk0 = 0; blk0 < p.k_blocks; blk0 += split) {
+			const int blk = blk0 + part;
+			const bool live = alone || blk < p.k_blocks;  // else a last round of fewer blocks than CTAs
 			// code and twiddle reads stay in the loop: held across it they spill
 			asm volatile("" : "+l"(code), "+l"(tw1), "+l"(tw2));
-			if (tid < NB0) {
+			if (live && tid < NB0) {
 				const float2* x = p.spectra + (static_cast<size_t>(d) * p.k_blocks + blk) * N + tid;
 				float2 v[R0];
 #pragma unroll
@@ -384,7 +467,7 @@ namespace ugsdr_gpu {
 					first[r] = v[r];
 			}
 			__syncthreads();
-			for (int u = tid; u < NB1; u += kSmallThreads) {  // u = k0 + R0 j1
+			for (int u = live ? tid : NB1; u < NB1; u += kSmallThreads) {  // u = k0 + R0 j1
 				const float2* w = tw1 + u % R0;
 				float2 v[R1];
 #pragma unroll
@@ -399,7 +482,10 @@ namespace ugsdr_gpu {
 					t[u + r * GS] = v[r];
 			}
 			__syncthreads();
-			if (tid < NB2) {
+			if (!alone && blk0)
+				add_round(blk0 - split, false);
+			odd = !odd;
+			if (live && tid < NB2) {
 				float2 v[R2];
 #pragma unroll
 				for (int r = 0; r < R2; ++r)
@@ -410,16 +496,31 @@ namespace ugsdr_gpu {
 				Dft<R2, true>::run(v);
 				float m[R2];
 				stats_of(v, scale, stat, m);
+				if constexpr (alone) {
 #pragma unroll
-				for (int r = 0; r < R2; ++r)
-					acc[tid + r * NB2] += m[r];
+					for (int r = 0; r < R2; ++r)
+						acc[tid + r * NB2] += m[r];
+				}
+				else {
+					float* const to = (odd ? mag : acc) + tid;
+#pragma unroll
+					for (int r = 0; r < R2; ++r)
+						to[r * NB2] = m[r];
+				}
 			}
+			if (!alone)
+				cluster_arrive();
 			__syncthreads();  // the next block's pass 0 rewrites the tile
 		}
-		if (plan.split > 1 && !cluster_sum(acc, N, plan.split, part))
-			return;
+		if (!alone) {
+			add_round((p.k_blocks - 1) / split * split, true);
+			cluster_arrive();
+			cluster_wait();
+			if (part != 0)
+				return;
+		}
 		__syncthreads();
-		reduce_cell(acc, N, p.cells + static_cast<size_t>(c) * p.n_doppler + p.d_base + d);
+		reduce_cell(alone || !odd ? acc : mag, N, p.cells + static_cast<size_t>(c) * p.n_doppler + p.d_base + d);
 	}
 
 	template <class K>
@@ -430,11 +531,12 @@ namespace ugsdr_gpu {
 
 	// the launch error, if any, is the runtime's last error
 	template <class K>
-	void launch_inv_small(K kernel, const AcqParams& p, const SmallPlan& plan, int rows, int smem, cudaStream_t stream) {
+	void launch_inv_small(K kernel, const AcqParams& p, const SmallPlan& plan, int rows, cudaStream_t stream) {
+		const int smem = small_inv_bytes(plan);
 		cudaLaunchConfig_t cfg{};
 		cfg.gridDim = dim3(static_cast<unsigned>(rows) * plan.split);
 		cfg.blockDim = dim3(plan.threads);
-		cfg.dynamicSmemBytes = smem;
+		cfg.dynamicSmemBytes = smem + small_cluster_bytes(plan);
 		cfg.stream = stream;
 		cudaLaunchAttribute cluster{};
 		cluster.id = cudaLaunchAttributeClusterDimension;
@@ -443,6 +545,6 @@ namespace ugsdr_gpu {
 		cfg.attrs = &cluster;
 		cfg.numAttrs = plan.split > 1 ? 1 : 0;
 		cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmallSmem);
-		cudaLaunchKernelEx(&cfg, kernel, p, plan);
+		cudaLaunchKernelEx(&cfg, kernel, p, plan, smem / static_cast<int>(sizeof(float)));
 	}
 }

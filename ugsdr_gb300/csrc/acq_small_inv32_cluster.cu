@@ -1,0 +1,8 @@
+// Single-CTA inverse kernel of clusters, one-sided spectra, radices up to 32.
+#include "acq_small.cuh"
+
+namespace ugsdr_gpu {
+	void launch_inv_small32_cluster(const AcqParams& p, const SmallPlan& plan, int rows, cudaStream_t stream) {
+		launch_inv_small(acq_inv_small_kernel<32, true, true>, p, plan, rows, stream);
+	}
+}
