@@ -475,13 +475,23 @@ namespace ugsdr_gpu {
 	// Inter-step twiddle seeds of the row stage, per CTA: for each of its rows
 	// k1 = r0 + f, W_N^{-j k1} for j < NS and W_N^{-NS k1} at j = NS, where NS
 	// is the stride of the plan's last pass (whose butterflies start at base
-	// = j < NS); built once per CTA and reused over the K blocks.
-	__device__ __forceinline__ void build_row_seeds(float2* seeds, int rows, int ns, int r0, uint32_t n) {
+	// = j < NS); built once per CTA and reused over the K blocks.  gain: factor
+	// on the transform, a power of two.
+	__device__ __forceinline__ void build_row_seeds(float2* seeds, int rows, int ns, int r0, uint32_t n, float gain = 1.0f) {
 		const float inv_n2 = 2.0f / static_cast<float>(n);
 		for (int e = threadIdx.x; e < rows * (ns + 1); e += blockDim.x) {
 			const int f = e / (ns + 1), j = e - f * (ns + 1);
-			seeds[e] = tw_n((static_cast<uint32_t>(j) * static_cast<uint32_t>(r0 + f)) % n, n, inv_n2, true);
+			const float2 w = tw_n((static_cast<uint32_t>(j) * static_cast<uint32_t>(r0 + f)) % n, n, inv_n2, true);
+			seeds[e] = j < ns ? cscale(w, gain) : w;
 		}
+	}
+	// The column kernels that square before they scale get B scaled by the power
+	// of two next to 1 / N, which changes no bit of the results but keeps the
+	// squares in range for samples of up to 1e14 (N^2 times the correlation
+	// overflows from 1e12 on at 40,920 points, from 1e10 on at 500,000).
+	__device__ __forceinline__ float row_gain(uint32_t n) { return __int_as_float((127 - (32 - __clz(n - 1))) << 23); }
+	__device__ __forceinline__ float column_scale(uint32_t n, int one_sided) {
+		return (one_sided ? 2.0f : 1.0f) / static_cast<float>(n) / row_gain(n);
 	}
 
 	struct InvRowsEmit {
@@ -632,7 +642,7 @@ namespace ugsdr_gpu {
 			const InvRowsLoadStagedN load{InvRowsLoadStaged{xs, cs, code}, n2};
 			// twiddle seeds after the pass tables (N2 entries)
 			float2* seeds = const_cast<float2*>(p2.tw) + F2::N;
-			build_row_seeds(seeds, rw, F2::kLastNS, r0, static_cast<uint32_t>(n));
+			build_row_seeds(seeds, rw, F2::kLastNS, r0, static_cast<uint32_t>(n), BCW > 0 ? row_gain(n) : 1.0f);
 			for (int blk = 0; blk < q.k_blocks; ++blk) {
 				cp_async_wait_all();
 				__syncthreads();  // this block's X (and the twiddle table) in shared memory
@@ -783,7 +793,7 @@ namespace ugsdr_gpu {
 		float2* cs = CODE ? xs + RPW * SL : nullptr;
 		const FftPlanDev p2 = F2::prepare(p.p2, smem + WARPS * WT);
 		float2* seeds = const_cast<float2*>(p2.tw) + N2;  // after the pass tables (N2 entries)
-		build_row_seeds(seeds, min(RW, n1 - rc), NS, rc, static_cast<uint32_t>(n));
+		build_row_seeds(seeds, min(RW, n1 - rc), NS, rc, static_cast<uint32_t>(n), row_gain(n));
 		__syncthreads();  // pass tables and seeds: the CTA's only barrier
 		if (rw == 0)
 			return;

@@ -123,8 +123,8 @@ namespace ugsdr_gpu {
 					acc[r] += m[r];
 			}
 		}
-		// scale once: |s y| = s |y| with s = 2 / N one-sided (1 / N two-sided)
-		const float s = (q.one_sided ? 2.0f : 1.0f) / static_cast<float>(q.n);
+		// scale once: |s y| = s |y| with s = 2 / N one-sided (1 / N two-sided), less the row stage's gain
+		const float s = column_scale(q.n, q.one_sided);
 		const float sc = STAT ? s * s : s;
 		const int n2g = chunk * P::CW + warp * P::CPW + c1;
 		MaxIdx best{-1.0f, 0xFFFFFFFFu};

@@ -248,27 +248,33 @@ namespace ugsdr_gpu {
 
 	// Sum and sum of squares, in double, of a thread's values.  Squares of
 	// magnitudes summed over K blocks cancel like (mean / sigma)^2 = 3.7 K in the
-	// variance, so floats sum only the deviations from a value a of the thread's
-	// own: sum v = n a + d and sum v^2 = sum (v - a)^2 + 2 a d + n a^2 hold for
-	// any a, and the smaller of two values is no correlation peak.  At 10,230
-	// points and K = 1,000 sigma is then within 4e-7 of 64 bits; float squares
-	// left 1.2e-5.
+	// variance, so floats sum only the deviations e = v / s - a from a value s a
+	// of the thread's own, s a power of two and 1 <= a < 2 (nothing leaves float's
+	// range): sum v = s (n a + sum e) and sum v^2 = s^2 (n a^2 + 2 a sum e + sum
+	// e^2) hold for any a, and the smaller of two values is no correlation peak.
+	// At 10,230 points and K = 1,000 sigma is then within 4e-7 of 64 bits; float
+	// squares left 1.2e-5.
 	struct Moments {
-		float a, d, m2;
+		float s, inv, a, d, m2;
 		int n;
-		__device__ __forceinline__ Moments(float v0, float v1) : a(fminf(v0, v1)), d(0.f), m2(0.f), n(0) {
-			if (!(a <= 3.4028234e38f))
-				a = 0.f;  // sums beyond float's range stay what they are
+		__device__ __forceinline__ Moments(float v0, float v1) : d(0.f), m2(0.f), n(0) {
+			const float v = fminf(v0, v1);
+			// (zeros, infinities and NaN: the values themselves)
+			const bool shift = v >= 1.17549435e-38f && v < 8.5070592e37f;
+			const int bits = shift ? __float_as_int(v) & 0x7F800000 : 0x3F800000;
+			s = __int_as_float(bits);
+			inv = __int_as_float(0x7F000000 - bits);
+			a = shift ? v * inv : 0.f;
 		}
 		__device__ __forceinline__ void add(float v) {
-			const float e = v - a;
+			const float e = fmaf(v, inv, -a);
 			d += e;
 			m2 = fmaf(e, e, m2);
 			++n;
 		}
-		__device__ __forceinline__ double sum() const { return static_cast<double>(n) * a + d; }
+		__device__ __forceinline__ double sum() const { return (static_cast<double>(n) * a + d) * s; }
 		__device__ __forceinline__ double squares() const {
-			return m2 + static_cast<double>(a) * (2.0 * d + static_cast<double>(n) * a);
+			return ((static_cast<double>(n) * a + 2.0 * d) * a + m2) * (static_cast<double>(s) * s);
 		}
 	};
 

@@ -106,7 +106,7 @@ namespace ugsdr_gpu {
 			const int k = e / (b1 - 1), r = e - k * (b1 - 1) + 1;
 			tw[k * lay.tws + r - 1] = __ldg(p.p2.tw + r * k);
 		}
-		build_row_seeds(seeds, rw, b0, r0, static_cast<uint32_t>(n));
+		build_row_seeds(seeds, rw, b0, r0, static_cast<uint32_t>(n), row_gain(n));
 		const float2* code = q.codes[c] + static_cast<size_t>(r0) * n2;
 		for (int f = 0; f < rw; ++f)
 			for (int e = threadIdx.x; e < lay.lds; e += blockDim.x)
@@ -266,8 +266,8 @@ namespace ugsdr_gpu {
 			});
 			__syncthreads();  // the next block's pass 0 rewrites the tile
 		}
-		// scale once: |s y| = s |y| with s = 2 / N one-sided (1 / N two-sided)
-		const float s = (q.one_sided ? 2.0f : 1.0f) / static_cast<float>(q.n);
+		// scale once: |s y| = s |y| with s = 2 / N one-sided (1 / N two-sided), less the row stage's gain
+		const float s = column_scale(q.n, q.one_sided);
 		const float sc = STAT ? s * s : s;
 		MaxIdx best{-1.0f, 0xFFFFFFFFu};
 		const float* const first = acc + threadIdx.x * lay.accs;
