@@ -242,12 +242,15 @@ namespace ugsdr_gpu {
 		// and the at most two groups that nulling touched.
 		__device__ __forceinline__ void detect_column(float* mag, float* group, const DetectScratch& d, size_t col, size_t cols,
 			int* s_hist, unsigned int* s_total) {
+			// maxima of bit patterns, which order as non-negative floats do and put a
+			// NaN above them all (a float maximum passes it over)
+			auto bits = [](float m) { return __float_as_uint(m); };
 			auto group_max = [&](int g) {
-				float m = mag[8 * g];
+				unsigned int m = bits(mag[8 * g]);
 #pragma unroll
 				for (int i = 1; i < 8; ++i)
-					m = fmaxf(m, mag[8 * g + i]);
-				group[g] = m;
+					m = max(m, bits(mag[8 * g + i]));
+				group[g] = __uint_as_float(m);
 			};
 #pragma unroll 4
 			for (int g = 0; g < 16; ++g)
@@ -256,20 +259,20 @@ namespace ugsdr_gpu {
 			float peaks[kMaxCandidates];
 #pragma unroll
 			for (int r = 0; r < kMaxCandidates; ++r) {
-				float top = group[0];
+				unsigned int top = bits(group[0]);
 				int g = 0;
 #pragma unroll
 				for (int i = 1; i < 16; ++i) {
-					const float m = group[i];
+					const unsigned int m = bits(group[i]);
 					g = m > top ? i : g;
-					top = fmaxf(top, m);
+					top = max(top, m);
 				}
 				int bi = 8 * g + 7;
 #pragma unroll
 				for (int i = 6; i >= 0; --i)
-					bi = mag[8 * g + i] == top ? 8 * g + i : bi;
+					bi = bits(mag[8 * g + i]) == top ? 8 * g + i : bi;
 				bins[r] = bi;
-				peaks[r] = top;
+				peaks[r] = __uint_as_float(top);
 #pragma unroll
 				for (int i = -kNullHalfWidth; i <= kNullHalfWidth; ++i)
 					mag[(bi + i) & (kDetectBins - 1)] = 0.0f;
