@@ -576,6 +576,7 @@ namespace ugsdr_gpu {
 				st->carrier_freq = carrier_freq;
 				st->carrier_phase_error = carrier_phase_error;
 				st->phase_fx = phase_fx;
+				st->phase_rad = phase_rad;
 				st->epoch += p.n_epochs;
 			}
 			if (threadIdx.x == 32) {
