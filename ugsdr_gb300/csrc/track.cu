@@ -100,9 +100,17 @@ namespace ugsdr_gpu {
 		}
 
 		// Named barriers of the loop update: one warp arrives, the others wait.
-		// Every participant reaches them once per epoch.
-		__device__ __forceinline__ void bar_arrive(int id, int threads) { asm volatile("bar.arrive %0, %1;\n" ::"r"(id), "r"(threads) : "memory"); }
-		__device__ __forceinline__ void bar_wait(int id, int threads) { asm volatile("bar.sync %0, %1;\n" ::"r"(id), "r"(threads) : "memory"); }
+		// Every participant reaches them once per epoch.  Both instructions are of
+		// the aligned kind, which a warp has to execute as one: it converges first,
+		// since lane-dependent branches and loops lead up to them.
+		__device__ __forceinline__ void bar_arrive(int id, int threads) {
+			__syncwarp();
+			asm volatile("bar.arrive %0, %1;\n" ::"r"(id), "r"(threads) : "memory");
+		}
+		__device__ __forceinline__ void bar_wait(int id, int threads) {
+			__syncwarp();
+			asm volatile("bar.sync %0, %1;\n" ::"r"(id), "r"(threads) : "memory");
+		}
 		constexpr int kBarFll = 1;     // warp 2 (FLL discriminator) -> warp 0
 		constexpr int kBarWindow = 2;  // warp 1 (tap set-up) -> warps 3.. (window copy)
 
@@ -545,7 +553,6 @@ namespace ugsdr_gpu {
 						prev_re = pr;
 						prev_im = pi;
 					}
-					__syncwarp();
 					bar_arrive(kBarFll, 64);
 				}
 				else {
