@@ -113,6 +113,7 @@ namespace ugsdr_gpu {
 	// Shape of one job as the large path needs it.
 	struct JobLaunchShape {
 		int n = 0, k = 0, m = 0, rows = 0, fold_mode = 0;
+		size_t slab = ScratchLimits{}.slab;
 	};
 
 	namespace {
@@ -449,15 +450,6 @@ namespace ugsdr_gpu {
 
 		int chunks_of(int total, int per) { return (total + per - 1) / per; }
 
-		// rows per inverse batch: B (rows x K x N complex) within 8 GiB — large
-		// enough that a batch is thousands of CTAs and a search a few hundred
-		// launches at most (the host then never waits on a full launch queue)
-		int batch_rows(const JobLaunchShape& s, size_t b_points) {
-			const size_t per_row = sizeof(float2) * b_points * s.k;
-			const size_t budget = static_cast<size_t>(8) << 30;
-			return static_cast<int>(std::max<size_t>(1, std::min<size_t>(s.rows, budget / per_row)));
-		}
-
 		template <typename K>
 		void launch_fwd_cols(ugsdr_ctx* ctx, K kernel, const BatchedParams& p, int items, int threads) {
 			const size_t smem = smem_cols(p);
@@ -525,6 +517,17 @@ namespace ugsdr_gpu {
 				}
 			}
 		};
+
+		// rows per inverse batch: B (rows x K x N complex) within 8 GiB — large
+		// enough that a batch is thousands of CTAs and a search a few hundred
+		// launches at most (the host then never waits on a full launch queue) —
+		// and the whole scratch within the job's limit, down to one row
+		int batch_rows(const JobLaunchShape& s, size_t b_points, int chunks) {
+			const size_t per_row = sizeof(float2) * b_points * s.k;
+			const size_t budget = static_cast<size_t>(8) << 30;
+			const size_t fit = s.slab / ScratchLayout(s, 1, chunks, b_points).total;
+			return static_cast<int>(std::max<size_t>(1, std::min({static_cast<size_t>(s.rows), budget / per_row, fit})));
+		}
 	}
 
 	// B points per (row, block) and column chunks per row of a job shape
@@ -548,7 +551,7 @@ namespace ugsdr_gpu {
 		int cwb = 0, chunks = 0;
 		size_t b_points = 0;
 		inverse_geometry(ctx, p, s.fold_mode, cwb, b_points, chunks);
-		return ScratchLayout(s, batch_rows(s, b_points), chunks, b_points).total;
+		return ScratchLayout(s, batch_rows(s, b_points, chunks), chunks, b_points).total;
 	}
 
 	void large_code_spectrum(ugsdr_ctx* ctx, CodeEntry& e, const float* chips_dev, size_t n_chips, size_t repeats,
@@ -620,7 +623,7 @@ namespace ugsdr_gpu {
 		p.row_keep = 0;
 		if (cw_blocked)
 			p.n2p = static_cast<int>(b_points / p.n1);
-		const int r_max = batch_rows(s, b_points);
+		const int r_max = batch_rows(s, b_points, chunks);
 		const ScratchLayout lay(s, r_max, chunks, b_points);
 		p.bbuf = reinterpret_cast<float2*>(scratch + lay.bbuf);
 		p.partials = reinterpret_cast<float4*>(scratch + lay.partials);
@@ -772,6 +775,7 @@ namespace ugsdr_gpu {
 		int folds = 1;        // F > 1: the block of F n samples is folded to n before the transforms
 		bool own_codes = false;  // code spectra of another length or layout than the handles'
 		float code_scale = 1.f;  // folded jobs: factor on the code spectra
+		ScratchLimits limits;
 		ResamplePlan rs{};
 	};
 
@@ -783,6 +787,7 @@ namespace ugsdr_gpu {
 			s.m = L.m;
 			s.rows = static_cast<int>(L.grid.size()) * L.n_codes;
 			s.fold_mode = L.fold_mode;
+			s.slab = L.limits.slab;
 			return s;
 		}
 
@@ -889,11 +894,12 @@ namespace ugsdr_gpu {
 		}
 	}
 
-	// Doppler bins per launch: mixed spectra (bins x K x N complex) within 4 GB
+	// Doppler bins per launch: mixed spectra (bins x K x N complex; a folded
+	// job's folded blocks, as many again, with them) within the job's limit
 	// (UGSDR_SPECTRA_BUDGET_MB overrides, e.g. to exercise chunking in tests).
 	int chunk_bins(const JobLaunch& L) {
-		const size_t per_bin = sizeof(float2) * static_cast<size_t>(L.n) * L.k;
-		size_t budget = static_cast<size_t>(4) << 30;
+		const size_t per_bin = sizeof(float2) * static_cast<size_t>(L.n) * L.k * (L.folds > 1 ? 2 : 1);
+		size_t budget = L.limits.spectra;
 		if (const char* env = std::getenv("UGSDR_SPECTRA_BUDGET_MB"))
 			budget = std::max<size_t>(1, std::strtoull(env, nullptr, 10)) << 20;
 		return static_cast<int>(std::max<size_t>(1, std::min<size_t>(L.grid.size(), budget / per_bin)));
@@ -1250,12 +1256,13 @@ namespace ugsdr_gpu {
 			return L.own_codes ? (sizeof(float2) * static_cast<size_t>(L.n) * L.n_codes + 255) / 256 * 256 : 0;
 		}
 
-		BatchSizes size_batch(ugsdr_ctx* ctx, const ugsdr_acq_job* jobs, int n_jobs) {
+		BatchSizes size_batch(ugsdr_ctx* ctx, const ugsdr_acq_job* jobs, int n_jobs, const ScratchLimits& limits = {}) {
 			require(jobs != nullptr && n_jobs >= 1, "no jobs");
 			BatchSizes s;
 			std::map<std::pair<const void*, size_t>, bool> seen;
 			for (int j = 0; j < n_jobs; ++j) {
 				s.launches.push_back(validate(ctx, jobs[j]));
+				s.launches.back().limits = limits;
 				const auto& L = s.launches.back();
 				if (!jobs[j].samples_on_device) {
 					const size_t bytes = job_bytes(jobs[j]);
@@ -1284,22 +1291,52 @@ namespace ugsdr_gpu {
 		};
 	}
 
-	size_t jobs_device_bytes(ugsdr_ctx* ctx, const ugsdr_acq_job* jobs, int n_jobs) {
-		const BatchSizes s = size_batch(ctx, jobs, n_jobs);
+	size_t jobs_device_bytes(ugsdr_ctx* ctx, const ugsdr_acq_job* jobs, int n_jobs, const ScratchLimits& limits) {
+		const BatchSizes s = size_batch(ctx, jobs, n_jobs, limits);
 		return s.samples + s.spectra + sizeof(AcqCellDev) * s.cells + s.params + s.slab + s.front + s.folded + s.fold_codes;
 	}
 
+	ScratchLimits fit_scratch(ugsdr_ctx* ctx, const ugsdr_acq_job* jobs, int n_jobs, size_t budget) {
+		ScratchLimits limits;
+		// what a buffer may take once the others have theirs: the row batches
+		// first, then (with single rows) the Doppler chunks
+		for (size_t ScratchLimits::*part : {&ScratchLimits::slab, &ScratchLimits::spectra}) {
+			const size_t all = jobs_device_bytes(ctx, jobs, n_jobs, limits);
+			if (all <= budget)
+				break;
+			limits.*part = 1;
+			const size_t least = jobs_device_bytes(ctx, jobs, n_jobs, limits);
+			if (least < budget) {
+				const BatchSizes s = size_batch(ctx, jobs, n_jobs, limits);
+				limits.*part = budget - least + (part == &ScratchLimits::slab ? s.slab : s.spectra + s.folded);
+			}
+		}
+		return limits;
+	}
+
 	EnqueuedBatch enqueue_jobs(ugsdr_ctx* ctx, Workspace& ws, cudaStream_t stream, const ugsdr_acq_job* jobs, int n_jobs,
-		void* host_cells) {
-		BatchSizes sizes = size_batch(ctx, jobs, n_jobs);
+		void* host_cells, const ScratchLimits& given) {
+		BatchSizes sizes = size_batch(ctx, jobs, n_jobs, given);
+		// no memory for the row batches: smaller ones, down to single rows
+		for (ScratchLimits limits = given; sizes.slab;) {
+			try {
+				ws.slab.reserve(sizes.slab);
+				break;
+			}
+			catch (const Error& e) {
+				limits.slab = sizes.slab / 4;
+				BatchSizes less = size_batch(ctx, jobs, n_jobs, limits);
+				if (e.status != UGSDR_E_NOMEM || less.slab >= sizes.slab)
+					throw;
+				sizes = std::move(less);
+			}
+		}
 		const std::vector<JobLaunch>& launches = sizes.launches;
 		const size_t params_b = sizes.params;
 		ws.samples.reserve(sizes.samples);
 		ws.spectra.reserve(sizes.spectra);
 		ws.cells.reserve(sizeof(AcqCellDev) * sizes.cells);
 		ws.params.reserve(params_b);
-		if (sizes.slab)
-			ws.slab.reserve(sizes.slab);
 		if (sizes.front)
 			ws.front.reserve(sizes.front);
 		if (sizes.folded)

@@ -274,12 +274,22 @@ namespace ugsdr_gpu {
 		std::vector<size_t> cell_offsets;          // per job, in cells
 		size_t n_cells = 0;
 	};
+	// What a batch's scratch may take, bytes: the row batches of the four-step
+	// inverse (beside their own limit of 8 GiB; a single row always) and the
+	// mixed spectra of one Doppler chunk (one bin always).  Fewer rows or bins
+	// per launch give the same results.
+	struct ScratchLimits {
+		size_t slab = ~static_cast<size_t>(0);
+		size_t spectra = static_cast<size_t>(4) << 30;
+	};
 	EnqueuedBatch enqueue_jobs(ugsdr_ctx* ctx, Workspace& ws, cudaStream_t stream, const ugsdr_acq_job* jobs, int n_jobs,
-		void* host_cells);
+		void* host_cells, const ScratchLimits& limits = {});
 	void finish_jobs(const EnqueuedBatch& b, const ugsdr_acq_job* jobs, int n_jobs, const void* host_cells,
 		ugsdr_acq_result* const* results, ugsdr_acq_cell* cells_out);
 	// Device bytes a batch needs beyond what `ws` already holds (admission control).
-	size_t jobs_device_bytes(ugsdr_ctx* ctx, const ugsdr_acq_job* jobs, int n_jobs);
+	size_t jobs_device_bytes(ugsdr_ctx* ctx, const ugsdr_acq_job* jobs, int n_jobs, const ScratchLimits& limits = {});
+	// Limits under which the batch needs at most `budget` bytes, where it can.
+	ScratchLimits fit_scratch(ugsdr_ctx* ctx, const ugsdr_acq_job* jobs, int n_jobs, size_t budget);
 
 	// capture framing (codes.cpp): bytes of a BBP DDC epoch at fs (0 if fs is not
 	// a whole number of kHz), bytes of n samples of any sample type (0 if the

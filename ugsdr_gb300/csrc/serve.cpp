@@ -79,6 +79,7 @@ namespace {
 		std::vector<int> codes;
 		std::vector<char> samples;  // host copy (empty for device-resident samples)
 		size_t estimate = 0;   // device bytes
+		ScratchLimits limits;  // under which they fit the server's budget
 		double work = 0;       // cell-blocks: codes x Doppler bins x N x K
 		std::chrono::steady_clock::time_point queued;
 		std::vector<ugsdr_acq_result> results;
@@ -337,7 +338,7 @@ struct ugsdr_server {
 				// estimated service); the slot's scratch follows the stream
 				free_slot->active = urgent ? free_slot->urgent : free_slot->stream;
 				free_slot->ws.set_stream(free_slot->active);
-				free_slot->batch = enqueue_jobs(ctx, free_slot->ws, free_slot->active, &job, 1, free_slot->cells.ptr);
+				free_slot->batch = enqueue_jobs(ctx, free_slot->ws, free_slot->active, &job, 1, free_slot->cells.ptr, r->limits);
 				UG_CUDA(cudaEventRecord(free_slot->event, free_slot->active));
 				if (trace)
 					std::fprintf(stderr, "[serve] %.1f admit ticket %llu work %.3g urgent %d enqueue %.1f ms\n", t_admit,
@@ -462,7 +463,8 @@ int ugsdr_server_submit(ugsdr_server* server, const ugsdr_acq_job* job, uint64_t
 			r->job.samples = r->samples.data();
 		}
 		std::lock_guard<std::mutex> lock(ctx->mutex);
-		r->estimate = jobs_device_bytes(ctx, &r->job, 1);  // validates the job too
+		r->limits = fit_scratch(ctx, &r->job, 1, server->budget);
+		r->estimate = jobs_device_bytes(ctx, &r->job, 1, r->limits);  // validates the job too
 		r->work = static_cast<double>(r->job.n_codes) * doppler_grid(r->job.doppler_range, r->job.doppler_step).size() *
 			static_cast<double>(r->job.block_samples) * static_cast<double>(r->job.n_blocks);
 	});
