@@ -288,6 +288,9 @@ namespace ugsdr_gpu {
 		ugsdr_acq_result* const* results, ugsdr_acq_cell* cells_out);
 	// Device bytes a batch needs beyond what `ws` already holds (admission control).
 	size_t jobs_device_bytes(ugsdr_ctx* ctx, const ugsdr_acq_job* jobs, int n_jobs, const ScratchLimits& limits = {});
+	// What a batch costs, in inverse transform points (of the folded length where
+	// the search folds first).
+	double jobs_work(ugsdr_ctx* ctx, const ugsdr_acq_job* jobs, int n_jobs);
 	// Limits under which the batch needs at most `budget` bytes, where it can.
 	ScratchLimits fit_scratch(ugsdr_ctx* ctx, const ugsdr_acq_job* jobs, int n_jobs, size_t budget);
 

@@ -80,7 +80,7 @@ namespace {
 		std::vector<char> samples;  // host copy (empty for device-resident samples)
 		size_t estimate = 0;   // device bytes
 		ScratchLimits limits;  // under which they fit the server's budget
-		double work = 0;       // cell-blocks: codes x Doppler bins x N x K
+		double work = 0;       // cell-blocks: codes x Doppler bins x N x K, N the length of the search's transforms
 		std::chrono::steady_clock::time_point queued;
 		std::vector<ugsdr_acq_result> results;
 		bool done = false;
@@ -465,8 +465,7 @@ int ugsdr_server_submit(ugsdr_server* server, const ugsdr_acq_job* job, uint64_t
 		std::lock_guard<std::mutex> lock(ctx->mutex);
 		r->limits = fit_scratch(ctx, &r->job, 1, server->budget);
 		r->estimate = jobs_device_bytes(ctx, &r->job, 1, r->limits);  // validates the job too
-		r->work = static_cast<double>(r->job.n_codes) * doppler_grid(r->job.doppler_range, r->job.doppler_step).size() *
-			static_cast<double>(r->job.block_samples) * static_cast<double>(r->job.n_blocks);
+		r->work = jobs_work(ctx, &r->job, 1);
 	});
 	if (st != UGSDR_OK)
 		return st;
