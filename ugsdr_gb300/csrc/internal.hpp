@@ -168,6 +168,7 @@ struct ugsdr_ctx {
 	std::map<int, std::unique_ptr<ugsdr_gpu::DevBuf>> twiddles;
 	std::map<int, ugsdr_gpu::FftPlanDesc> plans;
 	std::map<int, ugsdr_gpu::LargePlan> large_plans;
+	std::map<int, int> splits;  // per block size: the built-in four-step split (0: none)
 	std::map<int, std::unique_ptr<ugsdr_gpu::DevBuf>> pass_tables;  // single-CTA kernels: pass twiddles per size
 	std::map<int, ugsdr_gpu::TileChoice> tiles;  // per block size (ugsdr_tile_set / ugsdr_autotune)
 
