@@ -1296,8 +1296,8 @@ namespace ugsdr_gpu {
 	}
 
 	// a mixed sample and bin of a folded search against an inverse transform
-	// point: 0.8 ps to 4 - 5
-	constexpr double kFoldWork = 0.2;
+	// point: 0.52 ps (81 bins of two 1,000,000-point blocks, 85 us) to 4 - 5
+	constexpr double kFoldWork = 0.12;
 
 	size_t jobs_device_bytes(ugsdr_ctx* ctx, const ugsdr_acq_job* jobs, int n_jobs, const ScratchLimits& limits) {
 		const BatchSizes s = size_batch(ctx, jobs, n_jobs, limits);
