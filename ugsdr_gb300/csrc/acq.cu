@@ -803,10 +803,15 @@ namespace ugsdr_gpu {
 		// |y|), |.|^2 takes sqrt(F) off the code spectrum (F |y|^2 = |F y|^2 / F).
 		// Measured, 32 codes x 81 bins, F = 4 at 9.548 MHz: 2.70 -> 0.66 ms;
 		// 12 codes x 81 bins x 2 blocks, F = 20 at 50 MHz: 63.0 -> 0.83 ms.
+		// A thread of the mix adds its F samples in turn (0.185 us each) and M of
+		// them share a block, so that short folds of long blocks stay general: one
+		// code at one bin, 400,000 points to 100 410 us against 742, 40,000 to 50
+		// 124 against 184; to 200 102 against 87, 400,000 to 1,000 164 against 130.
+		constexpr int kLeastFolded = 128, kMostFolds = 512;
 		void fold_first(ugsdr_ctx* ctx, const ugsdr_acq_job& job, JobLaunch& L) {
 			const int f = L.n / L.m;
 			std::vector<int> r;
-			if (f < 2 || L.m < 2 || !plan_radices(L.m, r) || std::getenv("UGSDR_NO_FOLD_FIRST"))
+			if (f < 2 || f > kMostFolds || L.m < kLeastFolded || !plan_radices(L.m, r) || std::getenv("UGSDR_NO_FOLD_FIRST"))
 				return;
 			if (!fits_single_cta(ctx, L.m) && rule_split(ctx, L.m) == 0)
 				return;
