@@ -220,18 +220,25 @@ int ugsdr_doppler_bins(double range, double step, uint32_t* n);
 /* No counterpart in the reference (FFTW plans its own transforms): block
  * sizes above the single-CTA limit run as N = n1 x (N / n1) four-step
  * transforms, and these calls read, pin or tune the shape of one size.
+ * (Sizes from 5,700 points up to that limit run four-step with the built-in
+ * shape only; these calls refuse them as they do smaller ones.)
+ * The inverse of a split runs on one of three sets of kernels: warp-owned
+ * (200 x 250 and 400 x 500), pair (both halves products of two radices of 2 to
+ * 32, tiles of 4 or 8) or natural layout (any split, tiles of 1 to 8).
  * A shape changes the kernels' tiling and, through n1, the order of the
  * float sums: results agree with another shape's within float rounding,
  * and peaks and Doppler bins are the same on any signal above threshold. */
 typedef struct ugsdr_tile_shape {
 	int n1;          /* split (0 in ugsdr_tile_set: the built-in rule, the largest n1 <= sqrt N that fits) */
-	int cols;        /* columns per column-kernel CTA: 1, 2, 4 or 8 (0: rule) */
+	int cols;        /* columns per column-kernel CTA: 1, 2, 4 or 8 (0: rule; the warp-owned kernel has its own) */
 	int rows;        /* rows per row-kernel CTA: 1, 2, 4 or 8 (0: rule) */
-	int warp_cols;   /* 1: warp-owned column kernel where one is compiled for the split, 0: one tile of
-	                    `cols` columns per CTA, -1: rule (the warp-owned kernel where compiled) */
+	int warp_cols;   /* 1: the split's warp-owned or pair kernels where it has them (pair kernels: cols and rows of 1
+	                    or 2 count as 0), 0: natural layout, -1: rule (1, but cols or rows of 1 or 2 take a split of
+	                    the pair kernels to the natural layout) */
 	int warp_rows;   /* 1: warp-owned row kernel (with the warp-owned columns; each warp takes whole rows through
 	                    both passes, code rows staged), 2: the same with three rows per warp and the code rows read
-	                    through L1 / L2, 0: rows in CTA tiles of `rows` rows, -1: rule (1 where compiled) */
+	                    through L1 / L2, 0: rows in CTA tiles of `rows` rows, -1: rule (1 where compiled; the pair
+	                    and natural kernels have 0 only) */
 	int block_samples; /* N the shape is for (filled by ugsdr_tile_get / ugsdr_autotune, ignored by ugsdr_tile_set) */
 	double ms;       /* ugsdr_autotune: device time of the tuning search with this shape */
 } ugsdr_tile_shape;

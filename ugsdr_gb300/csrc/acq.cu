@@ -184,8 +184,10 @@ namespace ugsdr_gpu {
 		// 332,500 points; of the shapes measured for one split the fit's choice is
 		// 1.4 % (rows) and 3.4 % (columns) slower than the fastest on average.
 		// More than eight rows, or more than 192 threads, per row CTA were never
-		// the fastest.
-		PairPlan pair_plan(int n1, int n2) {
+		// the fastest.  cols, rows: the widths asked for (0, or one the kernels do
+		// not have: the fitted choice).
+		PairPlan pair_plan(int n1, int n2, int cols_wanted, int rows_wanted) {
+			auto wanted = [](int value, int wish) { return (wish != 4 && wish != 8) || value == wish; };
 			PairPlan best;
 			double best_cost = 1e300;
 			auto pairs = [](int n) {
@@ -199,6 +201,8 @@ namespace ugsdr_gpu {
 			auto regs = [](int x, int y) { return std::max(x, y) <= 25 ? 80 : 128; };
 			for (const int shift : {2, 3}) {
 				const int cw = 1 << shift;
+				if (!wanted(cw, cols_wanted))
+					continue;
 				PairPlan cols, rows;
 				double c_cols = 1e300, c_rows = 1e300;
 				for (const auto& [a0, a1] : pairs(n1))
@@ -217,7 +221,7 @@ namespace ugsdr_gpu {
 					}
 				for (const auto& [b0, b1] : pairs(n2))
 					for (const int rw : {4, 8})
-						for (int t = 32; t <= 192; t += 32) {
+						for (int t = wanted(rw, rows_wanted) ? 32 : 224; t <= 192; t += 32) {
 							const PairRows lay(b0, b1, rw, 1);
 							const PairRows full(b0, b1, rw, 0);
 							if (full.bytes > kPairSmem)
@@ -279,7 +283,7 @@ namespace ugsdr_gpu {
 		lp.p1 = get_plan(ctx, lp.n1);
 		lp.p2 = get_plan(ctx, lp.n2);
 		if (pairable(lp.n1) && pairable(lp.n2))
-			lp.pair = pair_plan(lp.n1, lp.n2);
+			lp.pair = t != ctx->tiles.end() ? pair_plan(lp.n1, lp.n2, t->second.cw, t->second.rw) : pair_plan(lp.n1, lp.n2, 0, 0);
 		return ctx->large_plans[n] = lp;
 	}
 
@@ -406,6 +410,11 @@ namespace ugsdr_gpu {
 			int cw = 0;
 			if (with_cols_warp(n1, n2, [&](auto plan) { cw = decltype(plan)::CW; }))
 				return cw;
+			// tiles of one or two columns or rows are the natural layout's, unless
+			// the pair kernels are asked for too
+			auto narrow = [](int width) { return width == 1 || width == 2; };
+			if (t != ctx->tiles.end() && t->second.warp_cols < 0 && (narrow(t->second.cw) || narrow(t->second.rw)))
+				return 0;
 			const PairPlan& pair = get_large_plan(ctx, n).pair;
 			return pair.a0 ? 1 << pair.cw_shift : 0;
 		}
@@ -1513,8 +1522,13 @@ namespace ugsdr_gpu {
 			t.n1 = lp.n1;
 			t.warp_cols = blocked_cw(ctx, n, lp.n1, lp.n2, 0) ? 1 : 0;
 			// the warp-owned row kernel runs with the warp-owned columns of the
-			// 200 x 250 and 400 x 500 splits
-			t.warp_rows = t.warp_cols ? warp_rows_mode(ctx, n) : 0;
+			// 200 x 250 and 400 x 500 splits; the pair kernels' rows are CTA tiles
+			const bool pairs = t.warp_cols && !has_static_plan(lp.n1, lp.n2);
+			t.warp_rows = t.warp_cols && !pairs ? warp_rows_mode(ctx, n) : 0;
+			if (pairs) {
+				t.cols = 1 << lp.pair.cw_shift;
+				t.rows = lp.pair.rw;
+			}
 			t.block_samples = n;
 			return t;
 		}
@@ -1555,7 +1569,7 @@ namespace ugsdr_gpu {
 
 		// Sets block size n's shape; an unusable shape leaves the old one.
 		void apply_tiles(ugsdr_ctx* ctx, int n, const TileChoice& t) {
-			require(!fits_single_cta(ctx, n), "block size runs on the single-CTA path (no four-step tiles)", UGSDR_E_INVALID);
+			require(!fits_single_cta(ctx, n), "block size within the single-CTA limit (no four-step tiles to set)", UGSDR_E_INVALID);
 			auto pow2 = [](int v) { return v == 0 || v == 1 || v == 2 || v == 4 || v == 8; };
 			require(pow2(t.cw) && pow2(t.rw) && t.warp_cols >= -1 && t.warp_cols <= 1 && t.warp_rows >= -1 && t.warp_rows <= 2,
 				"tile shape out of range");
@@ -1783,7 +1797,7 @@ int ugsdr_tile_get(ugsdr_ctx* ctx, size_t block_samples, ugsdr_tile_shape* shape
 		require(shape != nullptr, "null shape");
 		require(block_samples >= 2 && block_samples <= (1u << 24), "block size out of range");
 		const int n = static_cast<int>(block_samples);
-		require(!fits_single_cta(ctx, n), "block size runs on the single-CTA path (no four-step tiles)", UGSDR_E_INVALID);
+		require(!fits_single_cta(ctx, n), "block size within the single-CTA limit (no four-step tiles to set)", UGSDR_E_INVALID);
 		*shape = effective_shape(ctx, n);
 	});
 }
