@@ -472,16 +472,25 @@ namespace ugsdr_gpu {
 		const int zl = (zf + nb - 1) / nb * nb;
 		return zl < F2::N ? zl : F2::N;
 	}
+	// Products of a butterfly's inter-step twiddle recurrence before it starts
+	// again from its seed: the step's own rounding grows with their number (31 of
+	// them left 1e-6 of a twiddle at radix 32, 7 leave 2.4e-7)
+	constexpr int kTwiddleRun = 8;
+	constexpr int kTwiddleJumps = 3;  // restarts of the longest butterfly, radix 32
+
 	// Inter-step twiddle seeds of the row stage, per CTA: for each of its rows
 	// k1 = r0 + f, W_N^{-j k1} for j < NS and W_N^{-NS k1} at j = NS, where NS
 	// is the stride of the plan's last pass (whose butterflies start at base
 	// = j < NS); built once per CTA and reused over the K blocks.  gain: factor
-	// on the transform, a power of two.
-	__device__ __forceinline__ void build_row_seeds(float2* seeds, int rows, int ns, int r0, uint32_t n, float gain = 1.0f) {
+	// on the transform, a power of two.  jumps: that many powers 8, 16, ... of the
+	// last one beyond it (kTwiddleRun).
+	__device__ __forceinline__ void build_row_seeds(float2* seeds, int rows, int ns, int r0, uint32_t n, float gain = 1.0f, int jumps = 0) {
 		const float inv_n2 = 2.0f / static_cast<float>(n);
-		for (int e = threadIdx.x; e < rows * (ns + 1); e += blockDim.x) {
-			const int f = e / (ns + 1), j = e - f * (ns + 1);
-			const float2 w = tw_n((static_cast<uint32_t>(j) * static_cast<uint32_t>(r0 + f)) % n, n, inv_n2, true);
+		const int each = ns + 1 + jumps;
+		for (int e = threadIdx.x; e < rows * each; e += blockDim.x) {
+			const int f = e / each, j = e - f * each;
+			const uint32_t power = j <= ns ? j : kTwiddleRun * ns * (j - ns);
+			const float2 w = tw_n((power * static_cast<uint32_t>(r0 + f)) % n, n, inv_n2, true);
 			seeds[e] = j < ns ? cscale(w, gain) : w;
 		}
 	}

@@ -15,7 +15,7 @@
 // rows: L2), the code rows staged in shared memory once.  With one-sided
 // spectra (HALF) Z is zero from the middle of every row on, and pass 0 reads
 // b0 / 2 + 1 of its b0 inputs into the pruned DFT.  Pass 1 applies the
-// inter-step twiddle (seeds per row, a recurrence per butterfly) and stores B
+// inter-step twiddle (seeds per row, a recurrence of eight products per butterfly) and stores B
 // in the blocked layout B[n2 / CW][k1][n2 % CW].
 // Column stage (inv_cols_pair_kernel): a CTA takes CW columns of a row over
 // the K blocks; pass 0 reads its contiguous N1 x CW tile from global memory,
@@ -73,7 +73,7 @@ namespace ugsdr_gpu {
 			cs_at = static_cast<int>(sizeof(float2)) * ldb * rw;
 			tw_at = cs_at + static_cast<int>(sizeof(float2)) * lds * rw;
 			seeds_at = tw_at + static_cast<int>(sizeof(float2)) * tws * b0;
-			bytes = seeds_at + static_cast<int>(sizeof(float2)) * rw * (b0 + 1);
+			bytes = seeds_at + static_cast<int>(sizeof(float2)) * rw * (b0 + 1 + kTwiddleJumps);
 		}
 	};
 
@@ -106,7 +106,7 @@ namespace ugsdr_gpu {
 			const int k = e / (b1 - 1), r = e - k * (b1 - 1) + 1;
 			tw[k * lay.tws + r - 1] = __ldg(p.p2.tw + r * k);
 		}
-		build_row_seeds(seeds, rw, b0, r0, static_cast<uint32_t>(n), row_gain(n));
+		build_row_seeds(seeds, rw, b0, r0, static_cast<uint32_t>(n), row_gain(n), kTwiddleJumps);
 		const float2* code = q.codes[c] + static_cast<size_t>(r0) * n2;
 		for (int f = 0; f < rw; ++f)
 			for (int e = threadIdx.x; e < lay.lds; e += blockDim.x)
@@ -166,8 +166,12 @@ namespace ugsdr_gpu {
 					for (int r = 1; r < R; ++r)
 						v[r] = cmulc(v[r], wk[r]);
 					Dft<R, true>::run(v);
-					float2 w = seeds[f * (b0 + 1) + j];
-					const float2 step = seeds[f * (b0 + 1) + b0];
+					const float2* const sf = seeds + f * (b0 + 1 + kTwiddleJumps);
+					float2 w = sf[j];
+					const float2 step = sf[b0];
+					auto next = [&](int r) {  // the twiddle of output r + 1
+						w = (r + 1) % kTwiddleRun ? cmul(w, step) : cmul(sf[j], sf[b0 + (r + 1) / kTwiddleRun]);
+					};
 					float2* o = out + (f << cw_shift);
 					if ((b0 & cw_mask) == 0) {
 						// every output a fixed distance from the first
@@ -176,7 +180,7 @@ namespace ugsdr_gpu {
 #pragma unroll
 						for (int r = 0; r < R; ++r) {
 							o[r * inc] = cmul(v[r], w);
-							w = cmul(w, step);
+							next(r);
 						}
 					}
 					else {
@@ -184,7 +188,7 @@ namespace ugsdr_gpu {
 #pragma unroll
 						for (int r = 0; r < R; ++r) {
 							o[(i2 >> cw_shift) * chunk_elems + (i2 & cw_mask)] = cmul(v[r], w);
-							w = cmul(w, step);
+							next(r);
 							i2 += b0;
 						}
 					}

@@ -48,7 +48,7 @@ namespace ugsdr_gpu {
 		const PairCols lay(a0, a1, CW);
 		float2* const work = reinterpret_cast<float2*>(raw);
 		float2* const tw = reinterpret_cast<float2*>(raw + lay.tw_at);
-		float2* const seeds = reinterpret_cast<float2*>(raw + lay.acc_at);  // [column][a0 + 1]
+		float2* const seeds = reinterpret_cast<float2*>(raw + lay.acc_at);  // [column][a0 + 1 + kTwiddleJumps]
 		for (int i = threadIdx.x; i < 80; i += blockDim.x)
 			lut[i] = q.lut[i];
 		const int chunks = (n2 + CW - 1) / CW;
@@ -59,11 +59,14 @@ namespace ugsdr_gpu {
 			const int k = e / (a1 - 1), r = e - k * (a1 - 1) + 1;
 			tw[k * lay.tws + r - 1] = __ldg(p.p1.tw + r * k);
 		}
-		// W_N^{(c0 + c) j}, j < a0, and the recurrence's step W_N^{(c0 + c) a0}
+		// W_N^{(c0 + c) j}, j < a0, the recurrence's step W_N^{(c0 + c) a0} and its
+		// restarts
 		const float inv_n2 = 2.0f / static_cast<float>(q.n);
-		for (int e = threadIdx.x; e < CW * (a0 + 1); e += blockDim.x) {
-			const int c = e / (a0 + 1), j = e - c * (a0 + 1);
-			seeds[e] = tw_n((static_cast<uint32_t>(j) * static_cast<uint32_t>(c0 + c)) % n, n, inv_n2, false);
+		constexpr int J = kTwiddleJumps;
+		for (int e = threadIdx.x; e < CW * (a0 + 1 + J); e += blockDim.x) {
+			const int c = e / (a0 + 1 + J), j = e - c * (a0 + 1 + J);
+			const uint32_t power = j <= a0 ? j : kTwiddleRun * a0 * (j - a0);
+			seeds[e] = tw_n((power * static_cast<uint32_t>(c0 + c)) % n, n, inv_n2, false);
 		}
 		__syncthreads();
 		const int it1 = min(items, (group + 1) * per);
@@ -128,13 +131,14 @@ namespace ugsdr_gpu {
 					for (int r = 1; r < R; ++r)
 						v[r] = cmul(v[r], wk[r]);
 					Dft<R, false>::run(v);
-					float2 w = seeds[c * (a0 + 1) + j];
-					const float2 step = seeds[c * (a0 + 1) + a0];
+					const float2* const sc = seeds + c * (a0 + 1 + J);
+					float2 w = sc[j];
+					const float2 step = sc[a0];
 					float2* o = out + static_cast<size_t>(j) * n2 + c;
 #pragma unroll
 					for (int r = 0; r < R; ++r) {
 						*o = cmul(v[r], w);
-						w = cmul(w, step);
+						w = (r + 1) % kTwiddleRun ? cmul(w, step) : cmul(sc[j], sc[a0 + (r + 1) / kTwiddleRun]);
 						o += inc;
 					}
 				}
@@ -146,7 +150,7 @@ namespace ugsdr_gpu {
 	template <int ST>
 	void launch_fwd_cols_pair(const BatchedParams& p, int items, int sm_count, cudaStream_t stream) {
 		const PairCols lay(p.pair.a0, p.pair.a1, 8);
-		const int seeds = lay.acc_at + static_cast<int>(sizeof(float2)) * 8 * (p.pair.a0 + 1);
+		const int seeds = lay.acc_at + static_cast<int>(sizeof(float2)) * 8 * (p.pair.a0 + 1 + kTwiddleJumps);
 		const int parts = (p.n2 + 7) / 8, per = pair_items(items, parts, sm_count);
 		const int grid = (items + per - 1) / per * parts;
 		auto kernel = max(p.pair.a0, p.pair.a1) <= 25 ? fwd_cols_pair_kernel<ST, 25> : fwd_cols_pair_kernel<ST, 32>;
