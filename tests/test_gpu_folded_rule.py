@@ -11,7 +11,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("n,m,first", [(4000, 2, False), (4000, 100, False), (4000, 125, False), (4096, 128, True), (40000, 50, False),
                                        (40000, 200, True), (65536, 128, True), (131072, 128, False), (140000, 280, True),
-                                       (166400, 320, False), (38192, 9548, True)])
+                                       (166400, 320, False), (38192, 9548, True), (614400, 1024, True), (2046000, 2046, True)])
 def test_folds_first_where_the_mix_is_short(ctx, golden_codes, monkeypatch, n, m, first):
     from ugsdr_gb300 import _lib as L
     chips = unpack_codes(golden_codes, "gps_l1ca")

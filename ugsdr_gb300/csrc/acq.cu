@@ -816,11 +816,13 @@ namespace ugsdr_gpu {
 		// them share a block, so that short folds of long blocks stay general: one
 		// code at one bin, 400,000 points to 100 410 us against 742, 40,000 to 50
 		// 124 against 184; to 200 102 against 87, 400,000 to 1,000 164 against 130.
-		constexpr int kLeastFolded = 128, kMostFolds = 512;
+		// (From a thousand samples on the block's own transforms outgrow the chain
+		// at any number of folds.)
+		constexpr int kLeastFolded = 128, kMostFolds = 512, kLongFolded = 1000;
 		void fold_first(ugsdr_ctx* ctx, const ugsdr_acq_job& job, JobLaunch& L) {
 			const int f = L.n / L.m;
 			std::vector<int> r;
-			if (f < 2 || f > kMostFolds || L.m < kLeastFolded || !plan_radices(L.m, r) || std::getenv("UGSDR_NO_FOLD_FIRST"))
+			if (f < 2 || L.m < kLeastFolded || (f > kMostFolds && L.m < kLongFolded) || !plan_radices(L.m, r) || std::getenv("UGSDR_NO_FOLD_FIRST"))
 				return;
 			if (!fits_single_cta(ctx, L.m) && rule_split(ctx, L.m) == 0)
 				return;
