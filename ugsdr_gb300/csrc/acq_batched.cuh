@@ -952,8 +952,7 @@ namespace ugsdr_gpu {
 			const int f = div_fft_n<F1>(e, inv_n1);
 			return acc[f * ld + e - f * n1];
 		};
-		const int e_last = cw * n1 - 1;
-		Moments own(value(min(static_cast<int>(threadIdx.x), e_last)), value(min(static_cast<int>(threadIdx.x + blockDim.x), e_last)));
+		Moments own(static_cast<int>(threadIdx.x) < cw * n1 ? value(threadIdx.x) : __int_as_float(0x7F800000));
 		for (int e = threadIdx.x; e < cw * n1; e += blockDim.x) {
 			const int f = div_fft_n<F1>(e, inv_n1), i1 = e - f * n1;
 			const float v = acc[f * ld + i1];
@@ -961,12 +960,11 @@ namespace ugsdr_gpu {
 			best = better(best, cand);
 			own.add(v);
 		}
-		double dsum = own.sum(), dsq = own.squares();
+		double dsum = 0.0, dsq = 0.0;
+		own.reduce(&dsum, &dsq);
 		for (int o = 16; o > 0; o >>= 1) {
 			const MaxIdx other{__shfl_down_sync(0xffffffffu, best.v, o), __shfl_down_sync(0xffffffffu, best.i, o)};
 			best = better(best, other);
-			dsum += __shfl_down_sync(0xffffffffu, dsum, o);
-			dsq += __shfl_down_sync(0xffffffffu, dsq, o);
 		}
 		const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 		if (lane == 0) {

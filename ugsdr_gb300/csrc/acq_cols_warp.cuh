@@ -128,7 +128,7 @@ namespace ugsdr_gpu {
 		const float sc = STAT ? s * s : s;
 		const int n2g = chunk * P::CW + warp * P::CPW + c1;
 		MaxIdx best{-1.0f, 0xFFFFFFFFu};
-		Moments own(acc[0] * sc, acc[1] * sc);
+		Moments own(n2g < n2 ? acc[0] * sc : __int_as_float(0x7F800000));
 		if (n2g < n2) {
 #pragma unroll
 			for (int r = 0; r < P::R1; ++r) {  // n1 increases with r: strict > keeps the first maximum
@@ -140,12 +140,11 @@ namespace ugsdr_gpu {
 				own.add(v);
 			}
 		}
-		double dsum = own.sum(), dsq = own.squares();
+		double dsum = 0.0, dsq = 0.0;
+		own.reduce(&dsum, &dsq);
 		for (int o = 16; o > 0; o >>= 1) {
 			const MaxIdx other{__shfl_down_sync(0xffffffffu, best.v, o), __shfl_down_sync(0xffffffffu, best.i, o)};
 			best = better(best, other);
-			dsum += __shfl_down_sync(0xffffffffu, dsum, o);
-			dsq += __shfl_down_sync(0xffffffffu, dsq, o);
 		}
 		if (lane == 0) {
 			s_max[warp] = best;

@@ -246,25 +246,35 @@ namespace ugsdr_gpu {
 		return a;
 	}
 
-	// Sum and sum of squares, in double, of a thread's values.  Squares of
-	// magnitudes summed over K blocks cancel like (mean / sigma)^2 = 3.7 K in the
-	// variance, so floats sum only the deviations e = v / s - a from a value s a
-	// of the thread's own, s a power of two and 1 <= a < 2 (nothing leaves float's
-	// range): sum v = s (n a + sum e) and sum v^2 = s^2 (n a^2 + 2 a sum e + sum
-	// e^2) hold for any a, and the smaller of two values is no correlation peak.
-	// At 10,230 points and K = 1,000 sigma is then within 4e-7 of 64 bits; float
-	// squares left 1.2e-5.
+	// Sum and sum of squares of a warp's values.  Squares of magnitudes summed
+	// over K blocks cancel like (mean / sigma)^2 = 3.7 K in the variance, so floats
+	// sum only the deviations e = v / s - a from a value s a of the warp's own, s
+	// a power of two and 1 <= a < 2 (nothing leaves float's range): sum v = s (n a
+	// + sum e) and sum v^2 = s^2 (n a^2 + 2 a sum e + sum e^2) hold for any a (the
+	// nearer the mean the better: not that of a correlation peak).  At 10,230
+	// points and K = 1,000 sigma is then within 4e-7 of 64 bits; float squares
+	// left 1.2e-5.  The lanes' sums are joined as floats and turned into doubles
+	// once per warp: a lane's own doubles, at two lanes per clock and SM, cost
+	// 40,920-point searches of ten blocks 0.5 %.
 	struct Moments {
 		float s, inv, a, d, m2;
 		int n;
-		__device__ __forceinline__ Moments(float v0, float v1) : d(0.f), m2(0.f), n(0) {
-			const float v = fminf(v0, v1);
+		// v: a value of the lane's own, infinity in a lane without any
+		__device__ __forceinline__ explicit Moments(float v) : d(0.f), m2(0.f), n(0) {
+			// their mean, those beyond twice the smallest (and the missing ones)
+			// counted as the smallest
+			const unsigned int low = __reduce_min_sync(0xffffffffu, __float_as_uint(v));
+			float mean = v <= 2.0f * __uint_as_float(low) ? v : __uint_as_float(low);
+#pragma unroll
+			for (int o = 16; o > 0; o >>= 1)
+				mean += __shfl_xor_sync(0xffffffffu, mean, o);
+			mean *= 0.03125f;
 			// (zeros, infinities and NaN: the values themselves)
-			const bool shift = v >= 1.17549435e-38f && v < 8.5070592e37f;
-			const int bits = shift ? __float_as_int(v) & 0x7F800000 : 0x3F800000;
-			s = __int_as_float(bits);
-			inv = __int_as_float(0x7F000000 - bits);
-			a = shift ? v * inv : 0.f;
+			const bool shift = low >= 0x00800000u && low < 0x7B800000u;
+			const unsigned int bits = shift ? __float_as_uint(mean) & 0x7F800000u : 0x3F800000u;
+			s = __uint_as_float(bits);
+			inv = __uint_as_float(0x7F000000u - bits);
+			a = shift ? mean * inv : 0.f;
 		}
 		__device__ __forceinline__ void add(float v) {
 			const float e = fmaf(v, inv, -a);
@@ -272,9 +282,19 @@ namespace ugsdr_gpu {
 			m2 = fmaf(e, e, m2);
 			++n;
 		}
-		__device__ __forceinline__ double sum() const { return (static_cast<double>(n) * a + d) * s; }
-		__device__ __forceinline__ double squares() const {
-			return ((static_cast<double>(n) * a + 2.0 * d) * a + m2) * (static_cast<double>(s) * s);
+		// lane 0's sums of the warp
+		__device__ __forceinline__ void reduce(double* sum, double* squares) {
+			n = __reduce_add_sync(0xffffffffu, n);
+#pragma unroll
+			for (int o = 16; o > 0; o >>= 1) {
+				d += __shfl_down_sync(0xffffffffu, d, o);
+				m2 += __shfl_down_sync(0xffffffffu, m2, o);
+			}
+			if ((threadIdx.x & 31) == 0) {
+				const double da = a, dd = d, ds = s, na = da * n;
+				*sum = (na + dd) * ds;
+				*squares = ((na + 2.0 * dd) * da + m2) * (ds * ds);
+			}
 		}
 	};
 

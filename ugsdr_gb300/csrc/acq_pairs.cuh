@@ -274,9 +274,7 @@ namespace ugsdr_gpu {
 		const float s = column_scale(q.n, q.one_sided);
 		const float sc = STAT ? s * s : s;
 		MaxIdx best{-1.0f, 0xFFFFFFFFu};
-		const float* const first = acc + threadIdx.x * lay.accs;
-		const bool any = threadIdx.x < CW * a0;
-		Moments own(any ? first[0] * sc : 0.f, any ? first[1] * sc : 0.f);
+		Moments own(threadIdx.x < CW * a0 && chunk * CW + threadIdx.x % CW < n2 ? acc[threadIdx.x * lay.accs] * sc : __int_as_float(0x7F800000));
 		for (int u = threadIdx.x; u < CW * a0; u += blockDim.x) {
 			const int j = u / CW, n2g = chunk * CW + u % CW;
 			if (n2g >= n2)
@@ -287,16 +285,15 @@ namespace ugsdr_gpu {
 				own.add(v);
 			}
 		}
-		double dsum = own.sum(), dsq = own.squares();
-		auto warp_reduce = [&] {
+		double dsum = 0.0, dsq = 0.0;
+		own.reduce(&dsum, &dsq);
+		auto reduce_max = [&] {
 			for (int o = 16; o > 0; o >>= 1) {
 				const MaxIdx other{__shfl_down_sync(0xffffffffu, best.v, o), __shfl_down_sync(0xffffffffu, best.i, o)};
 				best = better(best, other);
-				dsum += __shfl_down_sync(0xffffffffu, dsum, o);
-				dsq += __shfl_down_sync(0xffffffffu, dsq, o);
 			}
 		};
-		warp_reduce();
+		reduce_max();
 		const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
 		if (lane == 0) {
 			s_max[warp] = best;
@@ -332,7 +329,11 @@ namespace ugsdr_gpu {
 			dsum += sm.x;
 			dsq += sm.y;
 		}
-		warp_reduce();
+		reduce_max();
+		for (int o = 16; o > 0; o >>= 1) {
+			dsum += __shfl_down_sync(0xffffffffu, dsum, o);
+			dsq += __shfl_down_sync(0xffffffffu, dsq, o);
+		}
 		if (lane != 0)
 			return;
 		const int row = p.row0 + lrow;
