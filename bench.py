@@ -307,7 +307,7 @@ def run_ours(args, world, rank):
         key = ("n1", "cols", "rows", "warp_cols", "warp_rows")
         kept_ms = next((x["ms"] for x in tried if x["block_samples"] == n and all(x[k] == t[k] for k in key)), None)
         tiles[str(n)] = {"split": f"{t['n1']}x{n // t['n1']}", "cols": t["cols"], "rows": t["rows"],
-                         "column_kernel": "warp-owned" if t["warp_cols"] else "tile",
+                         "column_kernel": ("tile" if not t["warp_cols"] else "warp-owned" if t["warp_rows"] else "warp-owned or pair"),
                          "row_kernel": {0: "tile", 1: "warp-owned", 2: "warp-owned, 3 rows/warp, code via L2"}[t["warp_rows"]],
                          "shapes_timed": sum(1 for x in tried if x["block_samples"] == n),
                          "rule_ms": rule_ms, "kept_ms": kept_ms}
@@ -1190,7 +1190,7 @@ def run_observables(args, world, rank):
                 "d2h_bytes_per_step": units * 32 + 4 * n_ch * (1 + OBS_CAP),
                 "ms_per_step": t_e2e * 1e3},
         "gpu_launches": launches,
-        "roofline": {"bound": "hbm", "kernel": "observables (obs_sigma + obs_segsum + obs_emit)", "achieved": achieved,
+        "roofline": {"bound": "hbm", "kernel": "observables (obs_sums + obs_sigma + obs_emit)", "achieved": achieved,
                      "peak": hbm_peak, "unit": "GB/s", "frac": achieved / hbm_peak, "traffic": None,
                      "algorithmic_bytes_per_launch": top_bytes, "kernel_ms": per_launch,
                      "peak_source": "hbm_gbs of MEASURED_PEAKS.json"},

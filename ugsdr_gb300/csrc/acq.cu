@@ -1,5 +1,5 @@
 // Batched acquisition engine: FFT planning, code-spectrum cache, job launch.
-// Host side of the kernels in acq_kernels.cuh / acq_large.cuh; C entry points
+// Host side of the kernels in acq_*.cuh; C entry points
 // ugsdr_code_put / ugsdr_code_release / ugsdr_acquire / ugsdr_acquire_batch.
 #include "internal.hpp"
 #include "acq_kernels.cuh"
@@ -133,8 +133,8 @@ namespace ugsdr_gpu {
 
 	// The built-in split: the largest N1 <= sqrt(N) that fits with 4 columns
 	// per CTA; the largest sizes (beyond ~1.8e7 points) fall back to single
-	// columns.  0: none.  Searched once per size: it is asked for at every call
-	// (42 us of one folded to 20,460 points, 10 of one of 5,720).
+	// columns.  0: none.  Searched once per size: every call asks for it (58 us
+	// of one folded to 20,460 points, 28 of one of 5,720).
 	int rule_split(ugsdr_ctx* ctx, int n) {
 		const auto known = ctx->splits.find(n);
 		if (known != ctx->splits.end())

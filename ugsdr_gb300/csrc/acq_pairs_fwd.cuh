@@ -1,5 +1,6 @@
 // Forward four-step kernels of the pair splits (acq_pairs.cuh): signal items
-// only (code spectra and the per-op DFT keep fwd_cols_kernel / fwd_rows_kernel).
+// and the per-op DFT's whole signal, one item (code spectra keep
+// fwd_cols_kernel / fwd_rows_kernel).
 //
 // fwd_cols_pair_kernel: pass 0 loads, converts and mixes its samples straight
 // into the butterfly's registers (the row index steps by a1, the NCO holders
